@@ -13,6 +13,7 @@
 // In large waves of non-trivial scenes both queues are then sorted by where each ray starts and
 // its direction octant (a counting sort: keys counted in the shading launch, a scan, a scatter),
 // so that neighbouring lanes of the next traversal walk the same nodes.
+// Waves of few paths run whole paths in one launch instead (path_kernel).
 // The per-path logic is PathTracer::trace (src/render/path_tracer.cpp:153-366) in FP32 with the
 // reference's RNG stream layout; every path writes only its own state, so images do not depend
 // on scheduling. Radiance is kept per path and added to the pixels in sample order after the
@@ -450,12 +451,11 @@ struct ShadeStats {
 };
 
 template <bool BATCH, bool TWO>
-__device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin, ShadeStats& stats,
-                                     unsigned& error) {
+__device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin, uint32_t depth,
+                                     ShadeStats& stats, unsigned& error) {
     const WaveSegment*      g     = segment_of<BATCH>(a, path);
     const DeviceScene&      s     = scene_of<BATCH>(a, g);
     const IntegratorParams& p     = params_of<BATCH>(a, g);
-    const uint32_t          depth = a.bounce;
     const float4            d4    = a.st.ray_d[path];
     const f3                dir   = xyz(d4);
     const float4            beta4 = a.st.beta[path];
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(128, 5) shade_kernel(KernelArgs a) {
             }
             path                 = a.q.bins[bin * static_cast<size_t>(a.capacity) + (i - prefix[bin])];
             unsigned          e  = 0;
-            const ShadeResult r  = shade_surface<BATCH, TWO>(a, path, bin, stats, e);
+            const ShadeResult r  = shade_surface<BATCH, TWO>(a, path, bin, a.bounce, stats, e);
             note_error<BATCH>(segment_of<BATCH>(a, path), e, error);
             ext_key              = r.continue_path ? 0u : kNone;
             shadow_key           = r.shadow ? 0u : kNone;
@@ -685,6 +685,57 @@ __global__ void __launch_bounds__(128, 5) shade_kernel(KernelArgs a) {
             warp_append(ext_key, path, &nctr->ext, next, 0);
         }
     }
+    warp_add_stat(a.q.stats + kStatShadowRays, stats.shadow_rays);
+    warp_add_stat(a.q.stats + kStatScattering, stats.scattering);
+    warp_add_stat(a.q.stats + kStatRoulette, stats.roulette);
+    warp_add_stat(a.q.stats + kStatMedium, stats.medium);
+    if (error) {
+        atomicOr(a.q.error, error);
+    }
+}
+
+// ---- whole paths in one launch ----
+
+// A wave whose paths all fit on the device at once (path_lanes) runs in one launch: each lane
+// carries its path from the camera ray to its end with the wavefront's functions in the
+// wavefront's order (extension ray, the previous vertex's shadow ray, shading), so every path's
+// result is the wavefront's bit for bit. The path state stays in the path's records, which a wave
+// this small finds in L1 and L2.
+// The wavefront of such a wave is bound by its launches: two per bounce, each as long as its slowest
+// ray, with nothing to fill the SMs meanwhile. One lane per path waits only for its own. Call of
+// mr_render_device, wavefront and this (B200): 36-triangle box, depth 8, 16,384 paths 0.40 and
+// 0.24 ms, 65,536 paths 0.44 and 0.38 ms; 500k-triangle field, depth 12, 65,536 paths 1.46 and
+// 0.88 ms; two-level 200k-triangle scene, 65,536 paths 1.93 and 1.03 ms. With more paths than lanes
+// the wavefront's sorted, converged launches win (262,144 paths through the box: 0.60 against
+// 0.83 ms). Bound by the latency of one path's instructions and loads: 4 resident warps per
+// scheduler at 128 registers.
+template <bool MEDIA, bool TWO>
+__global__ void __launch_bounds__(128, 4) path_kernel(KernelArgs a, uint32_t count) {
+    const uint32_t path = blockIdx.x * blockDim.x + threadIdx.x;
+    TraceCounters  tc_ext{0, 0}, tc_shadow{0, 0};
+    ShadeStats     stats;
+    unsigned       error  = 0;
+    bool           alive  = path < count;
+    bool           shadow = false;  // the previous vertex's shadow ray is still to be traced
+    for (uint32_t depth = 0; __any_sync(0xffffffffu, alive || shadow); ++depth) {
+        uint32_t key = kNone;
+        if (alive) {
+            key = extend_item<MEDIA, TWO>(a, a.scene, path, true, tc_ext, error);
+        }
+        if (shadow) {
+            shadow_item<MEDIA, TWO>(a, a.scene, path, tc_shadow, error);
+        }
+        alive = shadow = false;
+        if (key != kNone) {  // the path ends at maximum_depth at the latest
+            const ShadeResult r = shade_surface<false, TWO>(a, path, static_cast<int>(key), depth, stats, error);
+            alive               = r.continue_path;
+            shadow              = r.shadow;
+        }
+    }
+    warp_add_stat(a.q.stats + kStatExtendBounds, tc_ext.bounds);
+    warp_add_stat(a.q.stats + kStatExtendTriangles, tc_ext.triangles);
+    warp_add_stat(a.q.stats + kStatShadowBounds, tc_shadow.bounds);
+    warp_add_stat(a.q.stats + kStatShadowTriangles, tc_shadow.triangles);
     warp_add_stat(a.q.stats + kStatShadowRays, stats.shadow_rays);
     warp_add_stat(a.q.stats + kStatScattering, stats.scattering);
     warp_add_stat(a.q.stats + kStatRoulette, stats.roulette);
@@ -949,6 +1000,7 @@ struct LaunchShape {
     int trace_blocks[4]  = {0, 0, 0, 0};  // by media + 2 * two_level
     int shade_blocks     = 0;
     int shade_blocks_two = 0;
+    uint32_t path_lanes[4] = {0, 0, 0, 0};  // largest wave of path_kernel, by media + 2 * two_level
 };
 
 LaunchShape& launch_shape() {
@@ -972,6 +1024,18 @@ LaunchShape& launch_shape() {
         shape.shade_blocks = sms * std::max(1, per);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, shade_kernel<false, true>, 128, 0);
         shape.shade_blocks_two = sms * std::max(1, per);
+        const auto lanes = [&](auto* kernel) {
+            int blocks = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, 128, 0);
+            return static_cast<uint32_t>(sms * std::max(1, blocks) * 128);
+        };
+        // With media half of them: a path that scatters is several times longer than one that
+        // leaves, and a full device of such paths waits longer for its last ones than the wavefront
+        // takes (65,536 paths in fog: 1.68 against 1.58 ms).
+        shape.path_lanes[0] = lanes(path_kernel<false, false>);
+        shape.path_lanes[1] = lanes(path_kernel<true, false>) / 2;
+        shape.path_lanes[2] = lanes(path_kernel<false, true>);
+        shape.path_lanes[3] = lanes(path_kernel<true, true>) / 2;
         device = current;
     }
     return shape;
@@ -1184,6 +1248,19 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
     const LaunchShape& shape = launch_shape();
     const bool         media = scene.d.medium_count > 0;
     const bool         two   = scene.d.two_level != 0;
+    const int          variant = (media ? 1 : 0) + (two ? 2 : 0);
+    // Kernel timing counts the wavefront's traversal launches, and the shadow capture reads its queue.
+    if (init.count <= shape.path_lanes[variant] && !init.capture && !kernel_timing().enabled.load()) {
+        a.q.staging = nullptr;  // no sort keys
+        switch (variant) {
+        case 0: path_kernel<false, false><<<blocks, 128, 0, stream>>>(a, init.count); break;
+        case 1: path_kernel<true, false><<<blocks, 128, 0, stream>>>(a, init.count); break;
+        case 2: path_kernel<false, true><<<blocks, 128, 0, stream>>>(a, init.count); break;
+        default: path_kernel<true, true><<<blocks, 128, 0, stream>>>(a, init.count); break;
+        }
+        MR_CUDA(cudaGetLastError());
+        return;
+    }
     // Large waves sort each bounce's extension rays by origin cell and direction; small ones
     // keep their order (the sort's fixed cost would outweigh the coherence it buys).
     const bool         ray_sort = ws.queues.staging != nullptr && init.count >= kRaySortMinPaths &&
@@ -1214,7 +1291,6 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
         }
         // The first shadow rays (queued by bounce 0's shading) are traced with bounce 1.
         a.occluded_out = bounce == 1 && init.capture ? init.capture->occluded : nullptr;
-        const int variant = (media ? 1 : 0) + (two ? 2 : 0);
         switch (variant) {
         case 0: trace_kernel<false, false, false><<<shape.trace_blocks[0], 128, 0, stream>>>(a); break;
         case 1: trace_kernel<true, false, false><<<shape.trace_blocks[1], 128, 0, stream>>>(a); break;

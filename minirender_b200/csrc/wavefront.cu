@@ -72,13 +72,16 @@ __device__ __forceinline__ void warp_add_stat(unsigned long long* stat, uint32_t
     }
 }
 
-__device__ __forceinline__ Pcg32 load_rng(const PathState& st, uint32_t path) {
-    const ulonglong2 r = st.rng[path];
-    return {r.x, r.y};
+// The RNG as a path's record holds it.
+__device__ __forceinline__ Pcg32 rng_of(float4 w) {
+    return {static_cast<uint64_t>(__float_as_uint(w.y)) << 32 | __float_as_uint(w.x),
+            static_cast<uint64_t>(__float_as_uint(w.w)) << 32 | __float_as_uint(w.z)};
 }
 
-__device__ __forceinline__ void store_rng(const PathState& st, uint32_t path, const Pcg32& r) {
-    st.rng[path] = make_ulonglong2(r.state, r.increment);
+__device__ __forceinline__ float4 rng_words(const Pcg32& r) {
+    return make_float4(__uint_as_float(static_cast<uint32_t>(r.state)), __uint_as_float(static_cast<uint32_t>(r.state >> 32)),
+                       __uint_as_float(static_cast<uint32_t>(r.increment)),
+                       __uint_as_float(static_cast<uint32_t>(r.increment >> 32)));
 }
 
 // The scene and integrator settings of a path: the launch's own in a single-job wave, its
@@ -119,14 +122,10 @@ __device__ __forceinline__ void note_error(const WaveSegment* g, unsigned e, uns
 
 __device__ __forceinline__ void init_path(const KernelArgs& a, uint32_t slot, Pcg32 rng, f3 o, f3 d,
                                           float tmin, float tmax) {
-    a.st.rng[slot]      = make_ulonglong2(rng.state, rng.increment);
-    a.st.ray_o[slot]    = f4(o, tmin);
-    a.st.ray_d[slot]    = f4(d, tmax);
-    a.st.beta[slot]     = make_float4(1, 1, 1, 1);
-    a.st.radiance[slot] = make_float4(0, 0, 0, 0);
-    a.st.prev[slot]     = make_float4(0, 0, 0, 0);
-    a.st.flags[slot]    = 1u;  // previous_delta = true
-    a.q.ext[0][slot]    = slot;
+    store_pair(a.st.ray_o, slot, f4(o, tmin), f4(d, tmax));
+    store_pair(a.st.beta, slot, make_float4(1, 1, 1, 1), make_float4(0, 0, 0, kDeltaPdf));
+    store_pair(a.st.radiance, slot, make_float4(0, 0, 0, 0), rng_words(rng));
+    a.q.ext[0][slot] = slot;
 }
 
 // Stream derivation, film jitter and lens sample of one camera sample (PathTracer::sample_pixel,
@@ -262,9 +261,9 @@ __device__ __forceinline__ TraceResult trace_scene(const DeviceScene& s, const R
 template <bool MEDIA, bool TWO>
 __device__ __forceinline__ uint32_t extend_item(const KernelArgs& a, const DeviceScene& s, uint32_t path,
                                                 bool sorted, TraceCounters& tc, unsigned& error) {
-    const float4 o4 = a.st.ray_o[path];
-    const float4 d4 = a.st.ray_d[path];
-    RayQuery     q;
+    float4 o4, d4;
+    load_pair(a.st.ray_o, path, o4, d4);
+    RayQuery q;
     q.init(xyz(o4), xyz(d4));
     const TraceResult r    = trace_scene<false, TWO>(s, q, o4.w, d4.w, tc, error);
     uint32_t          kind = 0;
@@ -286,14 +285,14 @@ __device__ __forceinline__ uint32_t extend_item(const KernelArgs& a, const Devic
     if (MEDIA && s.medium_count > 0) {
         // MediumField::sample over [minimum, hit ? distance : maximum]
         // (src/render/path_tracer.cpp:170-177).
-        Pcg32  rng   = load_rng(a.st, path);
+        Pcg32  rng   = rng_of(a.st.rng[path]);
         float4 beta4 = a.st.beta[path];
         bool   scattered;
         float  scatter_t = 0, g = 0;
         const f3 w = field_sample(s, xyz(o4), xyz(d4), o4.w, r.slot != kNone ? r.t : d4.w, rng,
                                   scattered, scatter_t, g, error);
         f3 beta = xyz(beta4) * w;
-        store_rng(a.st, path, rng);
+        a.st.rng[path]  = rng_words(rng);  // not the sector: its shadow ray may be adding radiance
         a.st.beta[path] = f4(beta, beta4.w);
         if (!finite3(beta) || beta.x < 0 || beta.y < 0 || beta.z < 0) {
             error |= kErrorRadiance;
@@ -313,9 +312,9 @@ __device__ __forceinline__ uint32_t extend_item(const KernelArgs& a, const Devic
 template <bool MEDIA, bool TWO>
 __device__ __forceinline__ void shadow_item(const KernelArgs& a, const DeviceScene& s, uint32_t path,
                                             TraceCounters& tc, unsigned& error) {
-    const float4 o4 = a.st.shadow_o[path];
-    const float4 d4 = a.st.shadow_d[path];
-    RayQuery     q;
+    float4 o4, d4;
+    load_pair(a.st.shadow_o, path, o4, d4);
+    RayQuery q;
     q.init(xyz(o4), xyz(d4));
     const TraceResult r = trace_scene<true, TWO>(s, q, 0.0f, o4.w, tc, error);
     if (a.occluded_out) {
@@ -456,28 +455,27 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
     const WaveSegment*      g     = segment_of<BATCH>(a, path);
     const DeviceScene&      s     = scene_of<BATCH>(a, g);
     const IntegratorParams& p     = params_of<BATCH>(a, g);
-    const float4            d4    = a.st.ray_d[path];
+    float4                  o4, d4, beta4, prev4, L4, words;
+    load_pair(a.st.ray_o, path, o4, d4);
+    load_pair(a.st.beta, path, beta4, prev4);
+    load_pair(a.st.radiance, path, L4, words);
     const f3                dir   = xyz(d4);
-    const float4            beta4 = a.st.beta[path];
     f3                      beta  = xyz(beta4);
     float                   eta_scale = beta4.w;
-    const float4            prev4 = a.st.prev[path];
-    const bool              previous_delta = a.st.flags[path] & 1u;
-    float4                  L4    = a.st.radiance[path];
+    const bool              previous_delta = prev4.w < 0;
     f3                      L     = xyz(L4);
     ShadeResult             out{false, false, 0u, 0u};
 
     if (bin == kBinMiss) {
         L += beta * environment_radiance(s, dir) *
              emission_weight(p, depth, previous_delta, prev4.w, environment_pdf(s, dir));
-        a.st.radiance[path] = f4(L, 0);
+        store_pair(a.st.radiance, path, f4(L, 0), words);
         return out;
     }
-    Pcg32 rng = load_rng(a.st, path);
+    Pcg32 rng = rng_of(words);
     if (bin == kBinMedium) {
         // Medium vertex (src/render/path_tracer.cpp:178-223).
         const float4 h      = a.st.hit[path];
-        const float4 o4     = a.st.ray_o[path];
         const f3     vertex = xyz(o4) + h.x * dir;
         const float  g      = h.y;
         if (depth == p.maximum_depth) {
@@ -501,8 +499,7 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
                 if (p.mode == MR_SAMPLING_MIS && !ls.discrete) {
                     weight = power_heuristic(ls.probability, phase);
                 }
-                a.st.shadow_o[path] = f4(vertex, limit);
-                a.st.shadow_d[path] = f4(sd, 0);
+                store_pair(a.st.shadow_o, path, f4(vertex, limit), f4(sd, 0));
                 a.st.shadow_c[path] = f4(beta * ls.radiance * (phase * weight / ls.probability), 0);
                 out.shadow          = true;
                 out.shadow_sort_key = a.q.staging ? coherence_key(s, kNone, vertex, sd) : 0u;
@@ -513,30 +510,28 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
         ++stats.scattering;
         ++stats.medium;
         if (!roulette(p, depth, rng, beta, eta_scale, stats.roulette)) {
-            store_rng(a.st, path, rng);
             return out;
         }
-        a.st.prev[path]  = f4(vertex, pdf);
-        a.st.flags[path] = 0u;
-        a.st.ray_o[path] = f4(vertex, 0.0f);
-        a.st.ray_d[path] = f4(next, INFINITY);
-        a.st.beta[path]  = f4(beta, eta_scale);
-        store_rng(a.st, path, rng);
+        store_pair(a.st.ray_o, path, f4(vertex, 0.0f), f4(next, INFINITY));
+        store_pair(a.st.beta, path, f4(beta, eta_scale), f4(vertex, pdf));
+        store_pair(a.st.radiance, path, L4, rng_words(rng));
         out.continue_path = true;
         out.sort_key      = a.q.staging ? coherence_key(s, kNone, vertex, next) : 0u;
         return out;
     }
 
     // Surface vertex (src/render/path_tracer.cpp:224-363).
-    const float4     h   = a.st.hit[path];
-    const uint32_t   slot = a.st.hit_slot[path];
+    float4 h, hit_words;
+    load_pair(a.st.hit, path, h, hit_words);
+    const uint32_t   slot = __float_as_uint(hit_words.x);
     const SurfaceHit sh  = surface_hit<TWO>(s, dir, slot, h.y, h.z, h.w);
     const DeviceMaterial m = s.materials[sh.material];
     if (m.emission.x > 0 || m.emission.y > 0 || m.emission.z > 0) {
         L += beta * m.emission *
              emission_weight(p, depth, previous_delta, prev4.w,
                              area_pdf(s, xyz(prev4), sh.prim, sh.position));
-        a.st.radiance[path] = f4(L, 0);
+        L4 = f4(L, 0);
+        a.st.radiance[path] = L4;
     }
     if (depth == p.maximum_depth) {
         return out;
@@ -579,8 +574,7 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
                     if (p.mode == MR_SAMPLING_MIS && !ls.discrete) {
                         weight = power_heuristic(ls.probability, bsdf.pdf(wo, wi));
                     }
-                    a.st.shadow_o[path] = f4(origin, limit);
-                    a.st.shadow_d[path] = f4(sd, 0);
+                    store_pair(a.st.shadow_o, path, f4(origin, limit), f4(sd, 0));
                     a.st.shadow_c[path] = f4(beta * bsdf.evaluate(wo, wi) * wi.z * ls.radiance *
                                                  (weight / ls.probability),
                                              0);
@@ -592,13 +586,11 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
     }
     Bsdf::Sample sample;
     if (!bsdf.sample(wo, component, dux, duy, sample) || max3(sample.weight) == 0) {
-        store_rng(a.st, path, rng);
         return out;
     }
     const f3    wi_world = normalize(frame.to_world(sample.direction));
     const float sides    = dot(wo_world, sh.geometric_normal) * dot(wi_world, sh.geometric_normal);
     if ((sample.transmission && sides >= 0) || (!sample.transmission && sides <= 0)) {
-        store_rng(a.st, path, rng);
         return out;
     }
     beta = beta * sample.weight;
@@ -611,15 +603,11 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
     const f3 origin = offset_origin(sh.position, sh.geometric_normal, sh.position_error, wi_world);
     const f3 next   = normalize(wi_world);
     if (!roulette(p, depth, rng, beta, eta_scale, stats.roulette)) {
-        store_rng(a.st, path, rng);
         return out;
     }
-    a.st.prev[path]  = f4(sh.position, sample.probability);
-    a.st.flags[path] = sample.discrete ? 1u : 0u;
-    a.st.ray_o[path] = f4(origin, 0.0f);
-    a.st.ray_d[path] = f4(next, INFINITY);
-    a.st.beta[path]  = f4(beta, eta_scale);
-    store_rng(a.st, path, rng);
+    store_pair(a.st.ray_o, path, f4(origin, 0.0f), f4(next, INFINITY));
+    store_pair(a.st.beta, path, f4(beta, eta_scale), f4(sh.position, sample.discrete ? kDeltaPdf : sample.probability));
+    store_pair(a.st.radiance, path, L4, rng_words(rng));
     out.continue_path = true;
     out.sort_key      = a.q.staging ? coherence_key(s, slot, origin, next) : 0u;
     return out;

@@ -89,13 +89,33 @@ struct RecordField {
     __host__ __device__ explicit operator bool() const { return base != nullptr; }
 };
 
+// The two 16-byte fields of one 32-byte sector of a record, `lower` at its lower address, moved by
+// one access: half the instructions and load-store wavefronts of two 16-byte ones, and a sector is
+// written whole. With 16-byte accesses the launches that move whole records were bound by that, not
+// by DRAM (camera paths at 1.6 TB/s). 4.2M paths through the 36-triangle box: camera launch 330 ->
+// 146 us (3.7 TB/s), the shading launches of a frame 1.77 -> 1.59 ms; 261k-triangle room, 15.1M
+// paths: 1.26 -> 0.69 ms and 12.7 -> 10.7 ms (B200).
+template <size_t STRIDE>
+__device__ __forceinline__ void load_pair(const RecordField<float4, STRIDE>& lower, size_t i, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(lower.base + i * STRIDE)
+                 : "memory");
+}
+template <size_t STRIDE>
+__device__ __forceinline__ void store_pair(const RecordField<float4, STRIDE>& lower, size_t i, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(lower.base + i * STRIDE), "f"(a.x),
+                 "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 // Path state of `capacity` paths as records: one 128-byte path record and one 64-byte shadow
 // record per path slot. Kernels reach paths by slot in queue and bin order, which scatters the
 // slots; a record keeps what one kernel reads of a path in whole 32-byte sectors instead of a
 // 16-byte piece of a sector in each of a dozen arrays. Path record sectors: the ray (ray_o,
-// ray_d: what traversal reads), the hit (hit, hit_slot, flags, segment: what traversal writes),
+// ray_d: what traversal reads), the hit (hit, hit_slot, segment: what traversal writes),
 // throughput and previous vertex (beta, prev), radiance and RNG (radiance, rng). Shading reads
-// and writes the four; a shadow test reads the shadow record's ray and, when the segment is clear,
+// the four and writes all but the hit, one 32-byte access per sector; a shadow test reads the shadow record's ray and, when the segment is clear,
 // its contribution and the path's radiance sector.
 constexpr size_t kPathRecordBytes   = 128;
 constexpr size_t kShadowRecordBytes = 64;
@@ -105,17 +125,20 @@ using PathField = RecordField<T, kPathRecordBytes>;
 template <typename T>
 using ShadowField = RecordField<T, kShadowRecordBytes>;
 
+// prev.w of a path whose previous event was a delta event (or the camera): no density is negative.
+constexpr float kDeltaPdf = -1.0f;
+
 struct PathState {
     PathField<float4>     ray_o;     // origin, interval minimum                        (+0)
     PathField<float4>     ray_d;     // direction, interval maximum                     (+16)
     PathField<float4>     hit;       // distance, barycentrics (medium: distance, g)    (+32)
     PathField<uint32_t>   hit_slot;  // triangle slot, kNone on a miss                  (+48)
-    PathField<uint32_t>   flags;     // bit 0: previous event was delta                 (+52)
     PathField<uint32_t>   segment;   // multi-job waves: the path's wave segment        (+56)
     PathField<float4>     beta;      // throughput, eta scale                           (+64)
-    PathField<float4>     prev;      // previous scattering vertex, previous pdf        (+80)
+    PathField<float4>     prev;      // previous scattering vertex and its pdf, kDeltaPdf
+                                     // where that was a delta event or the camera     (+80)
     PathField<float4>     radiance;  // accumulated radiance                            (+96)
-    PathField<ulonglong2> rng;       // PCG state, increment                            (+112)
+    PathField<float4>     rng;       // PCG state, increment (low and high words)       (+112)
     ShadowField<float4>   shadow_o;  // shadow origin, segment limit                    (+0)
     ShadowField<float4>   shadow_d;  // shadow direction                                (+16)
     ShadowField<float4>   shadow_c;  // unoccluded contribution                         (+32)
@@ -127,7 +150,6 @@ struct PathState {
         ray_d.base    = paths + 16;
         hit.base      = paths + 32;
         hit_slot.base = paths + 48;
-        flags.base    = paths + 52;
         segment.base  = with_segment ? paths + 56 : nullptr;
         beta.base     = paths + 64;
         prev.base     = paths + 80;

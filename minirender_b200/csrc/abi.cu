@@ -125,14 +125,25 @@ __global__ void query_kernel(DeviceScene s, const mr_ray* rays, size_t count, in
         RayQuery     q;
         q.init(make(r.origin[0], r.origin[1], r.origin[2]),
                make(r.direction[0], r.direction[1], r.direction[2]));
+        const auto direction = [&] { return make(rays[i].direction[0], rays[i].direction[1], rays[i].direction[2]); };
         if (any_hit) {
-            const TraceResult t = s.two_level ? trace2<true>(s, q, r.minimum, r.maximum, tc, err)
-                                              : trace<true>(s, q, r.minimum, r.maximum, tc, err);
-            occluded[i]         = t.slot != kNone ? 1 : 0;
+            const uint32_t slot =
+                s.two_level ? trace2<true>(s, q, r.minimum, r.maximum, tc, err).slot
+                            : trace<true>(s, q, r.minimum, r.maximum, direction, tc, err).slot;
+            occluded[i] = slot != kNone ? 1 : 0;
         } else {
-            const TraceResult t = s.two_level ? trace2<false>(s, q, r.minimum, r.maximum, tc, err)
-                                              : trace<false>(s, q, r.minimum, r.maximum, tc, err);
-            mr_hit            h{};
+            TraceResult t;
+            if (s.two_level) {
+                t = trace2<false>(s, q, r.minimum, r.maximum, tc, err);
+            } else {
+                const NearestHit nearest = trace<false>(s, q, r.minimum, r.maximum, direction, tc, err);
+                t.t                      = nearest.t;
+                t.slot                   = nearest.slot;
+                if (nearest.slot != kNone) {
+                    hit_edges(s, q.triangle_ray(), nearest.slot, t.a, t.b, t.c, t.det, t.flags, t.prim);
+                }
+            }
+            mr_hit h{};
             h.primitive = kNone;
             if (t.slot != kNone) {
                 const float b0 = __fdiv_rn(t.a, t.det), b1 = __fdiv_rn(t.b, t.det),

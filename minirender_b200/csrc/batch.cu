@@ -748,7 +748,7 @@ class Server {
         MR_CUDA(cudaMemcpyAsync(h_errors_[stage], d_errors_, settings_.max_jobs * sizeof(unsigned),
                                 cudaMemcpyDeviceToHost, lane.stream));
         MR_CUDA(cudaEventRecord(rec.done, lane.stream));
-        const uint64_t launches = Engine::batch_wave_launches(depth, ray_sort);
+        const uint64_t launches = Engine::batch_wave_launches(depth, media, two, ray_sort);
         note_launches(launches);
         stats_.kernel_launches += launches;
         stats_.segments += n;

@@ -1,14 +1,23 @@
 // device_scene.cuh — the scene as it lives in HBM.
 //
 // Traversal data and shading data are separate streams, each an array of 16-byte records:
-//  - nodes:  8 float4 (128 B, one cache line) per 4-wide node collapsed from the binary SAH
-//            tree. One fetch serves up to four slab tests, so a ray needs about half as many
+//  - nodes:  12 float4 (192 B, six 32-byte sectors) per 4-wide node collapsed from the binary SAH
+//            tree. One visit serves up to four slab tests, so a ray needs about half as many
 //            dependent node fetches as on the binary tree.
-//              [0..5] = lo.x, hi.x, lo.y, hi.y, lo.z, hi.z of children 0..3 (x4 vectors;
-//                       unused children hold an empty box)
-//              [6]    = child refs (int bits): >= 0 wide node index; < 0 leaf whose triangles
-//                       occupy slots ~ref .. the slot flagged kTriLeafEnd
-//              [7].x  = number of children (int bits)
+//              sector 0..3 = the x and the y planes of children 0..3 that a ray meets first, for
+//                       each pair of direction signs: (lo.x lo.y) (hi.x lo.y) (lo.x hi.y)
+//                       (hi.x hi.y), two x4 vectors each. The ray's near planes are sector
+//                       sx + 2 sy (s = 1 where the direction is negative), its far planes the
+//                       sector opposite, 3 - (sx + 2 sy).
+//              sector 4, 5 = lo.z and hi.z, each followed by the child refs (int bits): >= 0 wide
+//                       node index; < 0 leaf whose triangles occupy slots ~ref .. the slot
+//                       flagged kTriLeafEnd; 0 no child (the root is nobody's child). The near
+//                       z planes are sector 4 + sz.
+//            Unused children hold an empty box. A ray reads four sectors, each with one 32-byte
+//            load, and selects nothing. The x and y planes are stored twice for it: one 128-byte
+//            line with every plane once takes seven 16-byte loads, or four and eight selects (room
+//            7% slower); 64 bytes with 8-bit planes takes two loads and 33 more instructions to
+//            decode them (room 3% slower, the 36-triangle box 16%, whose flat boxes get thick).
 //  - tris:   3 float4 per triangle slot, in leaf order (no index indirection during traversal):
 //              [0] = v0.xyz, flat primitive id (uint bits)
 //              [1] = v1.xyz, flags (uint bits: kTriSingleSided | kTriMirrored | kind << 8)
@@ -55,6 +64,27 @@ __device__ __forceinline__ f3 world_normal(const float* m, const float* n) {
     const float length2 = __fadd_rn(__fadd_rn(__fmul_rn(w.x, w.x), __fmul_rn(w.y, w.y)), __fmul_rn(w.z, w.z));
     const float inverse = __fdiv_rn(1.0f, __fsqrt_rn(length2));
     return {__fmul_rn(w.x, inverse), __fmul_rn(w.y, inverse), __fmul_rn(w.z, inverse)};
+}
+
+constexpr size_t kWideNode = 12;  // float4 per wide node
+
+// Writes one wide node from its children's boxes (lo/hi[axis][child]) and refs.
+__device__ __forceinline__ void write_wide_boxes(float4* o, const float (*lo)[4], const float (*hi)[4]) {
+    const float4 lx = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
+    const float4 hx = make_float4(hi[0][0], hi[0][1], hi[0][2], hi[0][3]);
+    const float4 ly = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
+    const float4 hy = make_float4(hi[1][0], hi[1][1], hi[1][2], hi[1][3]);
+    o[0]  = lx, o[1] = ly;
+    o[2]  = hx, o[3] = ly;
+    o[4]  = lx, o[5] = hy;
+    o[6]  = hx, o[7] = hy;
+    o[8]  = make_float4(lo[2][0], lo[2][1], lo[2][2], lo[2][3]);
+    o[10] = make_float4(hi[2][0], hi[2][1], hi[2][2], hi[2][3]);
+}
+__device__ __forceinline__ void write_wide_refs(float4* o, const int* ref) {
+    o[9]  = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]),
+                        __int_as_float(ref[3]));
+    o[11] = o[9];
 }
 
 enum TriFlags : unsigned {

@@ -99,17 +99,20 @@ __global__ void rebase_nodes_kernel(const float4* in, uint32_t count, uint32_t n
     if (k >= count) {
         return;
     }
-    for (int r = 0; r < 8; ++r) {
-        out[8 * static_cast<size_t>(k) + r] = in[8 * static_cast<size_t>(k) + r];
+    const float4* from = in + kWideNode * static_cast<size_t>(k);
+    float4*       to   = out + kWideNode * static_cast<size_t>(k);
+    for (size_t r = 0; r < kWideNode; ++r) {
+        to[r] = from[r];
     }
-    float4&    refs = out[8 * static_cast<size_t>(k) + 6];
-    int        r4[4] = {__float_as_int(refs.x), __float_as_int(refs.y), __float_as_int(refs.z),
-                        __float_as_int(refs.w)};
+    const float4 refs  = from[9];
+    int          r4[4] = {__float_as_int(refs.x), __float_as_int(refs.y), __float_as_int(refs.z),
+                          __float_as_int(refs.w)};
     for (int i = 0; i < 4; ++i) {
-        r4[i] = r4[i] >= 0 ? r4[i] + static_cast<int>(node_base) : ~(~r4[i] + static_cast<int>(slot_base));
+        if (r4[i] != 0) {  // 0: no child
+            r4[i] = r4[i] > 0 ? r4[i] + static_cast<int>(node_base) : ~(~r4[i] + static_cast<int>(slot_base));
+        }
     }
-    refs = make_float4(__int_as_float(r4[0]), __int_as_float(r4[1]), __int_as_float(r4[2]),
-                       __int_as_float(r4[3]));
+    write_wide_refs(to, r4);
 }
 
 // One thread per instance triangle: the flattening's world vertices, checked as the flattened
@@ -271,7 +274,7 @@ __global__ void refit_kernel(mr_bvh_node* nodes, uint32_t count, const uint32_t*
     }
 }
 
-// Rows 0..5 of a mesh's wide nodes from the refit binary tree (children kept from the collapse).
+// The boxes of a mesh's wide nodes from the refit binary tree (children kept from the collapse).
 __global__ void refit_wide_kernel(const mr_bvh_node* nodes, const int4* children, uint32_t count, float4* wide) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) {
@@ -286,11 +289,7 @@ __global__ void refit_wide_kernel(const mr_bvh_node* nodes, const int4* children
             hi[a][i] = c[i] < 0 ? -INFINITY : nodes[c[i]].maximum[a];
         }
     }
-    float4* o = wide + 8 * static_cast<size_t>(k);
-    for (int a = 0; a < 3; ++a) {
-        o[2 * a]     = make_float4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
-        o[2 * a + 1] = make_float4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
-    }
+    write_wide_boxes(wide + kWideNode * static_cast<size_t>(k), lo, hi);
 }
 
 unsigned grid(size_t n, unsigned block = 256) { return static_cast<unsigned>((n + block - 1) / block); }
@@ -395,7 +394,7 @@ void build_mesh_trees(Scene& scene, const mr_scene_desc& desc, cudaStream_t stre
         node_total += wides[m].count;
         slot_total += mt.triangles;
     }
-    t.blas_nodes.allocate(std::max<uint32_t>(1, node_total) * 8ull);
+    t.blas_nodes.allocate(std::max<uint32_t>(1, node_total) * kWideNode);
     t.blas_tris.allocate(std::max<uint32_t>(1, slot_total) * 3ull);
     for (uint32_t m = 0; m < desc.mesh_count; ++m) {
         MeshTree& mt = t.mesh[m];
@@ -412,7 +411,7 @@ void write_mesh_tree(Scene& scene, uint32_t m, const WideTree& wide, cudaStream_
     if (wide.count) {
         rebase_nodes_kernel<<<grid(wide.count), 256, 0, stream>>>(wide.nodes.ptr, wide.count, mt.node_base,
                                                                    mt.slot_base,
-                                                                   t.blas_nodes.ptr + 8ull * mt.node_base);
+                                                                   t.blas_nodes.ptr + kWideNode * mt.node_base);
     }
     float4* slots = t.blas_tris.ptr + 3ull * mt.slot_base;
     mesh_slots_kernel<<<grid(mt.triangles), 256, 0, stream>>>(t.positions.ptr + 3ull * t.position_offset[m],
@@ -612,7 +611,7 @@ void refit_mesh(Scene& scene, uint32_t mesh, const float* device_positions, cuda
     if (mt.wide_count) {
         refit_wide_kernel<<<grid(mt.wide_count, 128), 128, 0, stream>>>(mt.nodes.ptr, mt.wide_children.ptr,
                                                                    mt.wide_count,
-                                                                   t.blas_nodes.ptr + 8ull * mt.node_base);
+                                                                   t.blas_nodes.ptr + kWideNode * mt.node_base);
     }
     float4* slots = t.blas_tris.ptr + 3ull * mt.slot_base;
     mesh_slots_kernel<<<grid(mt.triangles), 256, 0, stream>>>(t.positions.ptr + 3ull * t.position_offset[mesh],

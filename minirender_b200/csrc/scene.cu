@@ -141,7 +141,7 @@ __global__ void collapse_count_kernel(const mr_bvh_node* nodes, const uint32_t* 
     interior_counts[k] = interior;
 }
 
-// Writes wide node `base + k`: children's boxes as six x4 vectors, refs, child count.
+// Writes wide node `base + k` (layout in device_scene.cuh).
 __global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* children, uint32_t count,
                                       const uint32_t* offsets, uint32_t base, uint32_t next_base,
                                       float4* wide, uint32_t* next_roots) {
@@ -153,8 +153,7 @@ __global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* chil
     const int  c[4] = {c4.x, c4.y, c4.z, c4.w};
     float      lo[3][4], hi[3][4];
     int        ref[4];
-    int        valid = 0;
-    uint32_t   rank  = 0;
+    uint32_t   rank = 0;
     for (int i = 0; i < 4; ++i) {
         if (c[i] < 0) {
             for (int a = 0; a < 3; ++a) {
@@ -176,16 +175,10 @@ __global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* chil
         } else {
             ref[i] = ~static_cast<int>(n.first);
         }
-        ++valid;
     }
-    float4* o = wide + 8 * static_cast<size_t>(base + k);
-    for (int a = 0; a < 3; ++a) {
-        o[2 * a]     = make_float4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
-        o[2 * a + 1] = make_float4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
-    }
-    o[6] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]),
-                       __int_as_float(ref[3]));
-    o[7] = make_float4(__int_as_float(valid), 0.0f, 0.0f, 0.0f);
+    float4* o = wide + kWideNode * (static_cast<size_t>(base) + k);
+    write_wide_boxes(o, lo, hi);
+    write_wide_refs(o, ref);
 }
 
 __global__ void interior_count_kernel(const mr_bvh_node* nodes, uint32_t count, uint32_t* total) {
@@ -376,7 +369,7 @@ WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t node_count, cudaSt
         out.hi[a] = root.maximum[a];
     }
     out.root_count = root.count;
-    out.nodes.allocate(std::max<uint32_t>(1, interior) * 8ull);
+    out.nodes.allocate(std::max<uint32_t>(1, interior) * kWideNode);
     out.children.allocate(std::max<uint32_t>(1, interior));
     if (interior == 0) {
         return out;

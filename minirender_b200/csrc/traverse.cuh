@@ -21,6 +21,13 @@ namespace mr {
 constexpr int      kStackSize  = 195;
 constexpr uint32_t kMaxVisits  = 1u << 16;  // node visits per ray before the query gives up
 
+// The part of a ray that the triangle test uses: origin, permutation and shear.
+struct TriangleRay {
+    f3    o;
+    int   kx, ky, kz;
+    float sx, sy, sz;
+};
+
 struct RayQuery {
     f3    o, d;
     float inv_lo[3];  // 1/d scaled down by 2^-20: near slab distances round toward the origin
@@ -29,6 +36,7 @@ struct RayQuery {
     int   kx, ky, kz;
     float sx, sy, sz;
 
+    __device__ __forceinline__ TriangleRay triangle_ray() const { return {o, kx, ky, kz, sx, sy, sz}; }
     __device__ __forceinline__ void init(f3 origin, f3 direction) {
         o = origin;
         d = direction;
@@ -77,22 +85,45 @@ __device__ __forceinline__ float slab_enter(const RayQuery& q, float4 xy, float 
     return enter <= leave ? enter : __int_as_float(0x7fffffff);
 }
 
-// Slab test of one child of a wide node from its near and far planes per axis (already chosen by
-// the ray's direction signs): the entry distance, or +inf when missed. A hit's entry is at most
-// `tmax` (leave <= tmax), and +inf is also what an unbounded entry means, so interior traversal
-// treats +inf as "no child" without a second comparison against the interval.
-__device__ __forceinline__ float slab_near_far(const RayQuery& q, float nx, float fx, float ny, float fy,
-                                               float nz, float fz, float tmin, float tmax) {
-    const float tnx = (nx - q.o.x) * q.inv_lo[0];
-    const float tfx = (fx - q.o.x) * q.inv_hi[0];
-    const float tny = (ny - q.o.y) * q.inv_lo[1];
-    const float tfy = (fy - q.o.y) * q.inv_hi[1];
-    const float tnz = (nz - q.o.z) * q.inv_lo[2];
-    const float tfz = (fz - q.o.z) * q.inv_hi[2];
-    const float enter = fmaxf(fmaxf(tmin, tnx), fmaxf(tny, tnz));
-    const float leave = fminf(fminf(tmax, tfx), fminf(tfy, tfz));
+// A 32-byte load (one sector of a wide node): half the load instructions, and half the L1
+// wavefronts of divergent lanes, that two 16-byte loads would take.
+__device__ __forceinline__ void load_sector(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// Slab planes of a wide node's four children, two children per packed FP32 operation: the
+// distances ((p - o) * inv) of four planes, each operation rounded as its scalar form is.
+__device__ __forceinline__ float4 plane_distances(float4 p, float neg_o, float inv) {
+    const float2 o2 = make_float2(neg_o, neg_o), i2 = make_float2(inv, inv);
+    const float2 a  = __fmul2_rn(__fadd2_rn(make_float2(p.x, p.y), o2), i2);
+    const float2 b  = __fmul2_rn(__fadd2_rn(make_float2(p.z, p.w), o2), i2);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Entry distance of a child box from the distances of its near and far planes, or +inf when the
+// ray misses it. A hit's entry is at most `tmax` (leave <= tmax), and +inf is also what an
+// unbounded entry means, so interior traversal treats +inf as "no child" without a second
+// comparison against the interval. fmaxf/fminf ignore the NaN of 0 * inf (origin on the slab plane
+// of a zero direction component).
+__device__ __forceinline__ float box_entry(float nx, float ny, float nz, float fx, float fy, float fz,
+                                           float tmin, float tmax) {
+    const float enter = fmaxf(fmaxf(tmin, nx), fmaxf(ny, nz));
+    const float leave = fminf(fminf(tmax, fx), fminf(fy, fz));
     return enter <= leave ? enter : __int_as_float(0x7f800000);
 }
+
+// Offsets (in float4) of the sectors a ray reads of a wide node (layout in device_scene.cuh).
+struct SectorOffsets {
+    int near_xy, near_z;
+    __device__ __forceinline__ void init(const bool* neg) {
+        near_xy = (neg[0] ? 2 : 0) + (neg[1] ? 4 : 0);
+        near_z  = neg[2] ? 10 : 8;
+    }
+    __device__ __forceinline__ int far_xy() const { return 6 - near_xy; }
+    __device__ __forceinline__ int far_z() const { return 18 - near_z; }
+};
 
 __device__ __forceinline__ void order2(float& ta, int& ra, float& tb, int& rb) {
     if (tb < ta) {
@@ -105,24 +136,67 @@ __device__ __forceinline__ void order2(float& ta, int& ra, float& tb, int& rb) {
     }
 }
 
+// A wide node against a ray: the children's refs and their entries, +inf where the ray misses the
+// child within [tmin, tmax] or there is none.
+struct NodeVisit {
+    int   r0, r1, r2, r3;
+    float t0, t1, t2, t3;
+    __device__ __forceinline__ void visit(const float4* n, SectorOffsets at, f3 neg_near, f3 neg_far,
+                                          const float* inv_lo, const float* inv_hi, float tmin, float tmax) {
+        float4 nx, ny, nz, fx, fy, rf;
+        load_sector(n + at.near_xy, nx, ny);
+        load_sector(n + at.near_z, nz, rf);
+        load_sector(n + at.far_xy(), fx, fy);
+        float4 fz = __ldg(n + at.far_z());
+        nx = plane_distances(nx, neg_near.x, inv_lo[0]);
+        ny = plane_distances(ny, neg_near.y, inv_lo[1]);
+        nz = plane_distances(nz, neg_near.z, inv_lo[2]);
+        fx = plane_distances(fx, neg_far.x, inv_hi[0]);
+        fy = plane_distances(fy, neg_far.y, inv_hi[1]);
+        fz = plane_distances(fz, neg_far.z, inv_hi[2]);
+        r0 = __float_as_int(rf.x), r1 = __float_as_int(rf.y), r2 = __float_as_int(rf.z), r3 = __float_as_int(rf.w);
+        t0 = box_entry(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, tmin, tmax);
+        t1 = box_entry(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, tmin, tmax);
+        t2 = box_entry(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, tmin, tmax);
+        t3 = box_entry(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, tmin, tmax);
+    }
+    __device__ __forceinline__ uint32_t children() const { return 2 + (r2 != 0 ? 1 : 0) + (r3 != 0 ? 1 : 0); }
+    // Nearest child first.
+    __device__ __forceinline__ void sort() {
+        order2(t0, r0, t1, r1);
+        order2(t2, r2, t3, r3);
+        order2(t0, r0, t2, r2);
+        order2(t1, r1, t3, r3);
+        order2(t1, r1, t2, r2);
+    }
+};
+
 __device__ __forceinline__ float permuted(f3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
+
+// Sheared vertices (x, y; z before the scale) and the three unnormalised edge functions of the
+// watertight triangle test.
+__device__ __forceinline__ void triangle_edges(const TriangleRay& q, f3 v0, f3 v1, f3 v2, float* x, float* y,
+                                               float* z, float& a, float& b, float& c) {
+    const f3 t0 = v0 - q.o, t1 = v1 - q.o, t2 = v2 - q.o;
+    z[0] = permuted(t0, q.kz), z[1] = permuted(t1, q.kz), z[2] = permuted(t2, q.kz);
+    x[0] = fmaf(-q.sx, z[0], permuted(t0, q.kx));
+    y[0] = fmaf(-q.sy, z[0], permuted(t0, q.ky));
+    x[1] = fmaf(-q.sx, z[1], permuted(t1, q.kx));
+    y[1] = fmaf(-q.sy, z[1], permuted(t1, q.ky));
+    x[2] = fmaf(-q.sx, z[2], permuted(t2, q.kx));
+    y[2] = fmaf(-q.sy, z[2], permuted(t2, q.ky));
+    a = difference_of_products(x[1], y[2], y[1], x[2]);
+    b = difference_of_products(x[2], y[0], y[2], x[0]);
+    c = difference_of_products(x[0], y[1], y[0], x[1]);
+}
 
 // Watertight triangle test (src/render/intersection.cpp:108-152) in FP32. On acceptance returns
 // the distance and the three unnormalised edge functions plus their sum (the determinant).
-__device__ __forceinline__ bool triangle_test(const RayQuery& q, f3 v0, f3 v1, f3 v2, float tmin,
+__device__ __forceinline__ bool triangle_test(const TriangleRay& q, f3 v0, f3 v1, f3 v2, float tmin,
                                               float tmax, float& t, float& ea, float& eb,
                                               float& ec, float& det) {
-    const f3 t0 = v0 - q.o, t1 = v1 - q.o, t2 = v2 - q.o;
-    const float z0 = permuted(t0, q.kz), z1 = permuted(t1, q.kz), z2 = permuted(t2, q.kz);
-    const float p0x = fmaf(-q.sx, z0, permuted(t0, q.kx));
-    const float p0y = fmaf(-q.sy, z0, permuted(t0, q.ky));
-    const float p1x = fmaf(-q.sx, z1, permuted(t1, q.kx));
-    const float p1y = fmaf(-q.sy, z1, permuted(t1, q.ky));
-    const float p2x = fmaf(-q.sx, z2, permuted(t2, q.kx));
-    const float p2y = fmaf(-q.sy, z2, permuted(t2, q.ky));
-    const float a = difference_of_products(p1x, p2y, p1y, p2x);
-    const float b = difference_of_products(p2x, p0y, p2y, p0x);
-    const float c = difference_of_products(p0x, p1y, p0y, p1x);
+    float px[3], py[3], pz[3], a, b, c;
+    triangle_edges(q, v0, v1, v2, px, py, pz, a, b, c);
     if ((a < 0 || b < 0 || c < 0) && (a > 0 || b > 0 || c > 0)) {
         return false;
     }
@@ -130,7 +204,7 @@ __device__ __forceinline__ bool triangle_test(const RayQuery& q, f3 v0, f3 v1, f
     if (determinant == 0) {
         return false;
     }
-    const float pz0 = z0 * q.sz, pz1 = z1 * q.sz, pz2 = z2 * q.sz;
+    const float pz0 = pz[0] * q.sz, pz1 = pz[1] * q.sz, pz2 = pz[2] * q.sz;
     const float distance = __fdiv_rn(a * pz0 + b * pz1 + c * pz2, determinant);
     if (!(distance >= tmin && distance <= tmax)) {
         return false;
@@ -139,17 +213,21 @@ __device__ __forceinline__ bool triangle_test(const RayQuery& q, f3 v0, f3 v1, f
     constexpr float g2 = 2.0f * 5.9604644775390625e-08f / (1.0f - 2.0f * 5.9604644775390625e-08f);
     constexpr float g3 = 3.0f * 5.9604644775390625e-08f / (1.0f - 3.0f * 5.9604644775390625e-08f);
     constexpr float g5 = 5.0f * 5.9604644775390625e-08f / (1.0f - 5.0f * 5.9604644775390625e-08f);
-    const float x = fmaxf(fmaxf(fabsf(p0x), fabsf(p1x)), fabsf(p2x));
-    const float y = fmaxf(fmaxf(fabsf(p0y), fabsf(p1y)), fabsf(p2y));
+    const float x = fmaxf(fmaxf(fabsf(px[0]), fabsf(px[1])), fabsf(px[2]));
+    const float y = fmaxf(fmaxf(fabsf(py[0]), fabsf(py[1])), fabsf(py[2]));
     const float z = fmaxf(fmaxf(fabsf(pz0), fabsf(pz1)), fabsf(pz2));
     const float error_x    = g5 * (x + z);
     const float error_y    = g5 * (y + z);
     const float error_edge = 2.0f * (g2 * x * y + error_y * x + error_x * y);
     const float edge       = fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c));
-    const float error_distance =
-        3.0f * (g3 * edge * z + error_edge * z + g3 * z * edge) / fabsf(determinant);
-    if (distance <= error_distance) {
-        return false;
+    const float error = 3.0f * (g3 * edge * z + error_edge * z + g3 * z * edge);
+    // distance <= error / |determinant|, with the division only where the products are within
+    // 2^-20 of each other (or not finite): elsewhere their rounding cannot change the answer.
+    const float scaled = distance * fabsf(determinant);
+    if (!(scaled > error * 1.00000095367431640625f && scaled < __int_as_float(0x7f800000) && scaled > 1e-30f)) {
+        if (distance <= error / fabsf(determinant)) {
+            return false;
+        }
     }
     t   = distance;
     ea  = a;
@@ -159,12 +237,20 @@ __device__ __forceinline__ bool triangle_test(const RayQuery& q, f3 v0, f3 v1, f
     return true;
 }
 
+// Hit of a two-level traversal: its distance, edge functions and instance.
 struct TraceResult {
     float    t;
-    uint32_t slot;  // triangle slot in leaf order (two-level scenes: the primitive), kNone: miss
+    uint32_t slot;  // the flat primitive id, kNone: miss
     uint32_t prim;
     float    a, b, c, det;
-    uint32_t flags;  // two-level scenes: the hit instance's flags
+    uint32_t flags;  // the hit instance's flags
+};
+
+// Nearest hit of a flattened traversal. The edge functions are not carried through the traversal:
+// hit_edges evaluates them again for the triangle that won, with the arithmetic that accepted it.
+struct NearestHit {
+    float    t;
+    uint32_t slot;  // triangle slot in leaf order, kNone: miss
 };
 
 struct TraceCounters {
@@ -172,18 +258,26 @@ struct TraceCounters {
     uint32_t triangles;
 };
 
-// Nearest hit (ANY_HIT = false) or occlusion (ANY_HIT = true) in [tmin, tmax].
-// Lanes of a warp traverse interior nodes together and postpone the first leaf they reach until
-// every active lane holds one (or has finished), then test leaves together: interior and leaf
-// work are not interleaved across lanes.
-template <bool ANY_HIT>
-__device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuery& q, float tmin,
-                                             float tmax, TraceCounters& counters,
-                                             unsigned& error) {
-    TraceResult result;
-    result.t    = tmax;
-    result.slot = kNone;
-    result.prim = kNone;
+// No further node: larger than any node index, so one unsigned comparison tells an interior node
+// from a leaf reference (negative) and from the end.
+constexpr int kNoNode = 0x7fffffff;
+constexpr int kDeepNode = 0x7ffffffe;  // stream.cuh: the next nodes are in the stack's local part
+constexpr int kPopNode  = 0x7ffffffd;  // stream.cuh: the next node is on the stack
+
+// Nearest hit (ANY_HIT = false) or occlusion (ANY_HIT = true) in [tmin, tmax] over the flattened
+// tree. Lanes of a warp traverse interior nodes together and postpone the first leaf they reach
+// until every active lane holds one (or has finished), then test leaves together: interior and
+// leaf work are not interleaved across lanes.
+//
+// What bounds it is the load-store pipe (one wavefront per divergent lane and load) and issue
+// slots, so a node visit is four 32-byte loads and packed arithmetic, and the state kept across
+// the loops is what the loops use: the hit is a distance and a slot, `direction()` fetches the
+// ray's direction again for the rare single-sided triangle, and the visit bound is the box-test
+// count.
+template <bool ANY_HIT, typename Direction>
+__device__ __forceinline__ NearestHit trace(const DeviceScene& s, const RayQuery& q, float tmin, float tmax,
+                                            Direction direction, TraceCounters& counters, unsigned& error) {
+    NearestHit result{tmax, kNone};
     if (!s.has_nodes) {
         return result;
     }
@@ -198,18 +292,20 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
     if (!(root_enter <= tmax)) {
         return result;
     }
-    int2     stack[kStackSize];
-    int      sp     = 0;
-    int      node   = s.root;  // next node to visit (interior >= 0, leaf < 0)
-    bool     alive  = true;    // `node` is valid
-    int      leaf   = 0;
-    bool     held   = false;   // a postponed leaf in `leaf`
-    uint32_t visits = 0;
-    const float inf = __int_as_float(0x7f800000);
-    // Node rows 0..5 are lo.x, hi.x, lo.y, hi.y, lo.z, hi.z of the four children: the near plane
-    // of an axis is its hi row when the direction is negative there.
-    const int near_x = q.neg[0] ? 1 : 0, near_y = q.neg[1] ? 3 : 2, near_z = q.neg[2] ? 5 : 4;
-    // Next stacked subtree that can still contain a nearer hit, or none.
+    int2        stack[kStackSize];
+    int         sp    = 0;
+    int         node  = s.root;  // next node: interior (>= 0) or leaf (< 0)
+    bool        alive = true;
+    int         leaf  = 0;       // a postponed leaf
+    bool        held  = false;
+    const float inf   = __int_as_float(0x7f800000);
+    const f3    neg_o = -q.o;
+    SectorOffsets at;
+    at.init(q.neg);
+    // Every node visit counts at least two box tests and each leaf reference was pushed by a
+    // visit, so bounding the count ends traversal on any tree.
+    const uint32_t bounds_limit = counters.bounds + 2 * kMaxVisits;
+    // Next stacked subtree that can still contain a nearer hit, or kNoNode.
     const auto pop = [&]() {
         while (sp > 0) {
             const int2 e = stack[--sp];
@@ -220,8 +316,6 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
         }
         alive = false;
     };
-    // Every pass of every loop below visits a node or tests a leaf, and both count against
-    // kMaxVisits, so traversal ends on any input.
     while (alive || held) {
         if (alive && node < 0 && !held) {  // a leaf to test next (also a root that is a leaf)
             leaf = node;
@@ -230,41 +324,30 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
         }
         // Interior phase.
         while (alive && node >= 0) {
-            if (++visits > kMaxVisits) {
+            NodeVisit v;
+            v.visit(s.nodes + kWideNode * static_cast<size_t>(node), at, neg_o, neg_o, q.inv_lo, q.inv_hi, tmin,
+                    result.t);
+            counters.bounds += v.children();
+            if (counters.bounds > bounds_limit) {
                 error |= kErrorVisits;
                 return result;
             }
-            const float4* n   = s.nodes + 8 * static_cast<size_t>(node);
-            const float4  nx  = __ldg(n + near_x), fx = __ldg(n + (near_x ^ 1));
-            const float4  ny  = __ldg(n + near_y), fy = __ldg(n + (near_y ^ 1));
-            const float4  nz  = __ldg(n + near_z), fz = __ldg(n + (near_z ^ 1));
-            const int4    ref = __ldg(reinterpret_cast<const int4*>(n + 6));
-            counters.bounds += static_cast<uint32_t>(__ldg(reinterpret_cast<const int*>(n + 7)));
-            float t0 = slab_near_far(q, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, tmin, result.t);
-            float t1 = slab_near_far(q, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, tmin, result.t);
-            float t2 = slab_near_far(q, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, tmin, result.t);
-            float t3 = slab_near_far(q, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, tmin, result.t);
-            int r0 = ref.x, r1 = ref.y, r2 = ref.z, r3 = ref.w;
-            order2(t0, r0, t1, r1);
-            order2(t2, r2, t3, r3);
-            order2(t0, r0, t2, r2);
-            order2(t1, r1, t3, r3);
-            order2(t1, r1, t2, r2);
-            if (t0 != inf) {
+            v.sort();
+            if (v.t0 != inf) {
                 if (sp > kStackSize - 3) {
                     error |= kErrorStack;
                     return result;
                 }
-                if (t3 != inf) {
-                    stack[sp++] = make_int2(r3, __float_as_int(t3));
+                if (v.t3 != inf) {
+                    stack[sp++] = make_int2(v.r3, __float_as_int(v.t3));
                 }
-                if (t2 != inf) {
-                    stack[sp++] = make_int2(r2, __float_as_int(t2));
+                if (v.t2 != inf) {
+                    stack[sp++] = make_int2(v.r2, __float_as_int(v.t2));
                 }
-                if (t1 != inf) {
-                    stack[sp++] = make_int2(r1, __float_as_int(t1));
+                if (v.t1 != inf) {
+                    stack[sp++] = make_int2(v.r1, __float_as_int(v.t1));
                 }
-                node = r0;
+                node = v.r0;
             } else {
                 pop();
             }
@@ -279,10 +362,6 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
         }
         // Leaf phase: the postponed leaf, then any leaf the lane now points at.
         while (held) {
-            if (++visits > kMaxVisits) {
-                error |= kErrorVisits;
-                return result;
-            }
             for (uint32_t slot = static_cast<uint32_t>(~leaf);; ++slot) {
                 const float4* tp = s.tris + 3 * static_cast<size_t>(slot);
                 const float4  a4 = __ldg(tp + 0);
@@ -291,24 +370,21 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
                 const unsigned flags = __float_as_uint(b4.w);
                 counters.triangles++;
                 float t, ea, eb, ec, det;
-                if (triangle_test(q, xyz(a4), xyz(b4), xyz(c4), tmin, result.t, t, ea, eb, ec,
+                if (triangle_test(q.triangle_ray(), xyz(a4), xyz(b4), xyz(c4), tmin, result.t, t, ea, eb, ec,
                                   det)) {
                     bool visible = true;
                     if (flags & kTriSingleSided) {
                         const f3 outward = cross(xyz(b4) - xyz(a4), xyz(c4) - xyz(a4));
-                        const float side = dot(q.d, outward);
+                        const float side = dot(direction(), outward);
                         visible = (flags & kTriMirrored) ? side > 0 : side < 0;
                     }
-                    const uint32_t prim = __float_as_uint(a4.w);
-                    if (visible && (t < result.t || (t == result.t && prim < result.prim) ||
-                                    result.slot == kNone)) {
+                    // t <= result.t here: nearer, or a tie, which goes to the lower primitive id.
+                    if (visible &&
+                        (t < result.t || result.slot == kNone ||
+                         __float_as_uint(a4.w) <
+                             __float_as_uint(__ldg(s.tris + 3 * static_cast<size_t>(result.slot)).w))) {
                         result.t    = t;
                         result.slot = slot;
-                        result.prim = prim;
-                        result.a    = ea;
-                        result.b    = eb;
-                        result.c    = ec;
-                        result.det  = det;
                         if (ANY_HIT) {
                             return result;
                         }
@@ -329,6 +405,19 @@ __device__ __forceinline__ TraceResult trace(const DeviceScene& s, const RayQuer
     return result;
 }
 
+// Edge functions and determinant of the triangle in `slot` for a ray that hit it: the values
+// triangle_test accepted.
+__device__ __forceinline__ void hit_edges(const DeviceScene& s, const TriangleRay& q, uint32_t slot, float& ea,
+                                          float& eb, float& ec, float& det, unsigned& flags, uint32_t& prim) {
+    const float4* tp = s.tris + 3 * static_cast<size_t>(slot);
+    const float4  a4 = __ldg(tp + 0), b4 = __ldg(tp + 1), c4 = __ldg(tp + 2);
+    float         z[3], x[3], y[3];
+    triangle_edges(q, xyz(a4), xyz(b4), xyz(c4), x, y, z, ea, eb, ec);
+    det   = ea + eb + ec;
+    flags = __float_as_uint(b4.w);
+    prim  = __float_as_uint(a4.w);
+}
+
 // ---- two-level scenes ----
 
 // The world ray mapped into an instance's object space (same parameter t: the direction is not
@@ -341,6 +430,8 @@ struct ObjectRay {
     float o_near[3], o_far[3];
     float inv_lo[3], inv_hi[3];
     bool  neg[3];
+    __device__ __forceinline__ f3 near_origin() const { return {o_near[0], o_near[1], o_near[2]}; }
+    __device__ __forceinline__ f3 far_origin() const { return {o_far[0], o_far[1], o_far[2]}; }
 };
 
 constexpr float kInstanceMarginScale = 1.9073486328125e-06f;  // 2^-19 = 32 FP32 unit roundoffs
@@ -370,19 +461,6 @@ __device__ __forceinline__ void object_ray(const DeviceInstance2& inst, const Ra
     }
 }
 
-__device__ __forceinline__ float object_slab(const ObjectRay& r, float nx, float fx, float ny, float fy,
-                                             float nz, float fz, float tmin, float tmax) {
-    const float tnx = (nx - r.o_near[0]) * r.inv_lo[0];
-    const float tfx = (fx - r.o_far[0]) * r.inv_hi[0];
-    const float tny = (ny - r.o_near[1]) * r.inv_lo[1];
-    const float tfy = (fy - r.o_far[1]) * r.inv_hi[1];
-    const float tnz = (nz - r.o_near[2]) * r.inv_lo[2];
-    const float tfz = (fz - r.o_far[2]) * r.inv_hi[2];
-    const float enter = fmaxf(fmaxf(tmin, tnx), fmaxf(tny, tnz));
-    const float leave = fminf(fminf(tmax, tfx), fminf(tfy, tfz));
-    return enter <= leave ? enter : __int_as_float(0x7f800000);
-}
-
 // Entry and exit of a world box, or false when the ray misses it within [tmin, tmax].
 __device__ __forceinline__ bool world_box(const RayQuery& q, const float* lo, const float* hi,
                                           float tmin, float tmax, float& enter, float& leave) {
@@ -395,30 +473,6 @@ __device__ __forceinline__ bool world_box(const RayQuery& q, const float* lo, co
     enter = fmaxf(fmaxf(tmin, nx), fmaxf(ny, nz));
     leave = fminf(fminf(tmax, fx), fminf(fy, fz));
     return enter <= leave;
-}
-
-// Wide-node children of `node` tested with `test(nx, fx, ny, fy, nz, fz)` (the near/far plane
-// rows picked by `near`), ordered nearest first. Returns the child count hit (<= 4) with refs and
-// entries in r[] / t[].
-template <typename Test>
-__device__ __forceinline__ void wide_children(const float4* nodes, int node, const int near[3],
-                                              Test test, float t[4], int r[4], uint32_t& bounds) {
-    const float4* n   = nodes + 8 * static_cast<size_t>(node);
-    const float4  nx  = __ldg(n + near[0]), fx = __ldg(n + (near[0] ^ 1));
-    const float4  ny  = __ldg(n + near[1]), fy = __ldg(n + (near[1] ^ 1));
-    const float4  nz  = __ldg(n + near[2]), fz = __ldg(n + (near[2] ^ 1));
-    const int4    ref = __ldg(reinterpret_cast<const int4*>(n + 6));
-    bounds += static_cast<uint32_t>(__ldg(reinterpret_cast<const int*>(n + 7)));
-    t[0] = test(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x);
-    t[1] = test(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y);
-    t[2] = test(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z);
-    t[3] = test(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w);
-    r[0] = ref.x, r[1] = ref.y, r[2] = ref.z, r[3] = ref.w;
-    order2(t[0], r[0], t[1], r[1]);
-    order2(t[2], r[2], t[3], r[3]);
-    order2(t[0], r[0], t[2], r[2]);
-    order2(t[1], r[1], t[3], r[3]);
-    order2(t[1], r[1], t[2], r[2]);
 }
 
 // A wide node's or a lone leaf's stack discipline: a stack of (ref, entry) pairs shared by the
@@ -455,7 +509,8 @@ __device__ __forceinline__ TraceResult trace2(const DeviceScene& s, const RayQue
     int      sp     = 0;
     uint32_t visits = 0;
     const float inf = __int_as_float(0x7f800000);
-    const int near_w[3] = {q.neg[0] ? 1 : 0, q.neg[1] ? 3 : 2, q.neg[2] ? 5 : 4};
+    SectorOffsets at_w;
+    at_w.init(q.neg);
     stack[sp++] = make_int2(s.root, __float_as_int(enter));
     while (sp > 0) {
         const int2 top = stack[--sp];
@@ -468,17 +523,16 @@ __device__ __forceinline__ TraceResult trace2(const DeviceScene& s, const RayQue
         }
         const int node = top.x;
         if (node >= 0) {  // instance-level interior node
-            float t[4];
-            int   r[4];
-            wide_children(s.nodes, node, near_w,
-                          [&](float nx, float fx, float ny, float fy, float nz, float fz) {
-                              return slab_near_far(q, nx, fx, ny, fy, nz, fz, tmin, result.t);
-                          },
-                          t, r, counters.bounds);
+            NodeVisit v;
+            v.visit(s.nodes + kWideNode * static_cast<size_t>(node), at_w, -q.o, -q.o, q.inv_lo, q.inv_hi, tmin, result.t);
+            counters.bounds += v.children();
+            v.sort();
             if (sp > kStackSize2 - 4) {
                 error |= kErrorStack;
                 return result;
             }
+            const int   r[4] = {v.r0, v.r1, v.r2, v.r3};
+            const float t[4] = {v.t0, v.t1, v.t2, v.t3};
             for (int k = 3; k >= 0; --k) {
                 if (t[k] != inf) {
                     stack[sp++] = make_int2(r[k], __float_as_int(t[k]));
@@ -495,7 +549,8 @@ __device__ __forceinline__ TraceResult trace2(const DeviceScene& s, const RayQue
             if (world_box(q, inst.lo, inst.hi, tmin, result.t, ienter, ileave)) {
                 ObjectRay ro;
                 object_ray(inst, q, ileave, ro);
-                const int near_o[3] = {ro.neg[0] ? 1 : 0, ro.neg[1] ? 3 : 2, ro.neg[2] ? 5 : 4};
+                SectorOffsets at_o;
+                at_o.init(ro.neg);
                 const int base = sp;
                 stack[sp++] = make_int2(inst.blas_root, __float_as_int(ienter));
                 while (sp > base) {
@@ -508,17 +563,16 @@ __device__ __forceinline__ TraceResult trace2(const DeviceScene& s, const RayQue
                         return result;
                     }
                     if (e.x >= 0) {  // mesh-level interior node
-                        float t[4];
-                        int   r[4];
-                        wide_children(s.blas_nodes, e.x, near_o,
-                                      [&](float nx, float fx, float ny, float fy, float nz, float fz) {
-                                          return object_slab(ro, nx, fx, ny, fy, nz, fz, tmin, result.t);
-                                      },
-                                      t, r, counters.bounds);
+                        NodeVisit v;
+                        v.visit(s.blas_nodes + kWideNode * static_cast<size_t>(e.x), at_o, -ro.near_origin(), -ro.far_origin(), ro.inv_lo, ro.inv_hi, tmin, result.t);
+                        counters.bounds += v.children();
+                        v.sort();
                         if (sp > kStackSize2 - 4) {
                             error |= kErrorStack;
                             return result;
                         }
+                        const int   r[4] = {v.r0, v.r1, v.r2, v.r3};
+                        const float t[4] = {v.t0, v.t1, v.t2, v.t3};
                         for (int k = 3; k >= 0; --k) {
                             if (t[k] != inf) {
                                 stack[sp++] = make_int2(r[k], __float_as_int(t[k]));
@@ -537,7 +591,7 @@ __device__ __forceinline__ TraceResult trace2(const DeviceScene& s, const RayQue
                         const f3 v2 = transform_point(inst.to_world, c4.x, c4.y, c4.z);
                         counters.triangles++;
                         float tt, ea, eb, ec, det;
-                        if (triangle_test(q, v0, v1, v2, tmin, result.t, tt, ea, eb, ec, det)) {
+                        if (triangle_test(q.triangle_ray(), v0, v1, v2, tmin, result.t, tt, ea, eb, ec, det)) {
                             bool visible = true;
                             if (inst.flags & kTriSingleSided) {
                                 const float side = dot(q.d, cross(v1 - v0, v2 - v0));

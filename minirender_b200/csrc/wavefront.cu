@@ -2,7 +2,7 @@
 //
 // One wave = up to `capacity` camera paths, their state in one 128-byte record per path. Each
 // bounce runs two persistent kernels:
-//   trace   nearest-hit traversal of the bounce's ray queue, classifying every path into a
+//   trace   streamed nearest-hit traversal of the bounce's ray queue, classifying every path into a
 //           material bin (miss, diffuse, conductor, mirror, dielectric, medium) with
 //           warp-aggregated appends (match_any + popc + one atomic per key per warp), then
 //           any-hit traversal of the previous bounce's shadow queue, adding the unoccluded
@@ -25,6 +25,7 @@
 
 #include "errors.hpp"
 #include "shading.cuh"
+#include "stream.cuh"
 #include "wavefront.cuh"
 
 namespace mr {
@@ -243,21 +244,56 @@ __global__ void init_rays_kernel(KernelArgs a, WaveInit w) {
 
 // ---- trace: this bounce's nearest-hit queue + the previous bounce's shadow queue ----
 
-// Nearest hit of one extension ray, its material bin (or kNone) and, with media, the
-// free-flight sample over the hit interval.
-// Nearest hit or occlusion in `s`: the flattened traversal, or (TWO) the two-level one when the
-// scene has two levels.
-template <bool ANY_HIT, bool TWO>
-__device__ __forceinline__ TraceResult trace_scene(const DeviceScene& s, const RayQuery& q, float tmin,
-                                                   float tmax, TraceCounters& tc, unsigned& error) {
-    if constexpr (TWO) {
-        if (s.two_level) {
-            return trace2<ANY_HIT>(s, q, tmin, tmax, tc, error);
-        }
-    }
-    return trace<ANY_HIT>(s, q, tmin, tmax, tc, error);
+// The material bin of a nearest hit of `kind`. Surface bins only group paths by material for the
+// shading launch; unsorted, every surface hit goes to the first.
+__device__ __forceinline__ uint32_t hit_bin(uint32_t slot, uint32_t kind, bool sorted) {
+    return slot == kNone ? kBinMiss : kBinDiffuse + (sorted ? kind : 0u);
 }
 
+// Stores a flattened traversal's nearest hit of path `path`; returns its material bin.
+__device__ __forceinline__ uint32_t store_hit(const KernelArgs& a, const DeviceScene& s, const TriangleRay& q,
+                                              uint32_t path, const NearestHit& r, bool sorted) {
+    unsigned flags = 0;
+    if (r.slot != kNone) {
+        float    ea, eb, ec, det;
+        uint32_t prim;
+        hit_edges(s, q, r.slot, ea, eb, ec, det, flags, prim);
+        a.st.hit[path] = make_float4(r.t, __fdiv_rn(ea, det), __fdiv_rn(eb, det), __fdiv_rn(ec, det));
+    }
+    a.st.hit_slot[path] = r.slot;
+    return hit_bin(r.slot, (flags >> 8) & 0xffu, sorted);
+}
+
+// MediumField::sample over [minimum, hit ? distance : maximum] (src/render/path_tracer.cpp:170-177) of
+// a scene with media: the path's bin after it, `bin` unless the path scatters or ends (kNone). `t` is
+// the end of the interval.
+__device__ __forceinline__ uint32_t sample_media(const KernelArgs& a, const DeviceScene& s, uint32_t path,
+                                                 float4 o4, float4 d4, float t, uint32_t bin, unsigned& error) {
+    Pcg32  rng   = rng_of(a.st.rng[path]);
+    float4 beta4 = a.st.beta[path];
+    bool   scattered;
+    float  scatter_t = 0, g = 0;
+    const f3 w    = field_sample(s, xyz(o4), xyz(d4), o4.w, t, rng, scattered, scatter_t, g, error);
+    const f3 beta = xyz(beta4) * w;
+    a.st.rng[path]  = rng_words(rng);  // not the sector: in one launch its shadow ray may add radiance
+    a.st.beta[path] = f4(beta, beta4.w);
+    if (!finite3(beta) || beta.x < 0 || beta.y < 0 || beta.z < 0) {
+        error |= kErrorRadiance;
+        return kNone;
+    }
+    if (max3(beta) == 0) {
+        return kNone;
+    }
+    if (scattered) {
+        a.st.hit[path] = make_float4(scatter_t, g, 0, 0);
+        return kBinMedium;
+    }
+    return bin;
+}
+
+// Nearest hit of one extension ray, its material bin (or kNone) and, with media, the
+// free-flight sample over the hit interval. A scene is traversed flattened or (TWO, where it has
+// two levels) two-level.
 template <bool MEDIA, bool TWO>
 __device__ __forceinline__ uint32_t extend_item(const KernelArgs& a, const DeviceScene& s, uint32_t path,
                                                 bool sorted, TraceCounters& tc, unsigned& error) {
@@ -265,50 +301,49 @@ __device__ __forceinline__ uint32_t extend_item(const KernelArgs& a, const Devic
     load_pair(a.st.ray_o, path, o4, d4);
     RayQuery q;
     q.init(xyz(o4), xyz(d4));
-    const TraceResult r    = trace_scene<false, TWO>(s, q, o4.w, d4.w, tc, error);
-    uint32_t          kind = 0;
-    if (r.slot != kNone) {
-        a.st.hit[path] = make_float4(r.t, __fdiv_rn(r.a, r.det), __fdiv_rn(r.b, r.det),
-                                     __fdiv_rn(r.c, r.det));
-        if (sorted) {
-            if (TWO && s.two_level) {
-                kind = (r.flags >> 8) & 0xffu;
-            } else {
-                kind = (__float_as_uint(__ldg(s.tris + 3 * static_cast<size_t>(r.slot) + 1).w) >> 8) & 0xffu;
-            }
+    uint32_t bin;
+    float    t;
+    if (TWO && s.two_level) {
+        const TraceResult r = trace2<false>(s, q, o4.w, d4.w, tc, error);
+        if (r.slot != kNone) {
+            a.st.hit[path] = make_float4(r.t, __fdiv_rn(r.a, r.det), __fdiv_rn(r.b, r.det),
+                                         __fdiv_rn(r.c, r.det));
         }
+        a.st.hit_slot[path] = r.slot;
+        bin                 = hit_bin(r.slot, (r.flags >> 8) & 0xffu, sorted);
+        t                   = r.t;
+    } else {
+        const NearestHit r =
+            trace<false>(s, q, o4.w, d4.w, [&] { return xyz(a.st.ray_d[path]); }, tc, error);
+        bin = store_hit(a, s, q.triangle_ray(), path, r, sorted);
+        t   = r.t;
     }
-    a.st.hit_slot[path] = r.slot;
-    // Surface bins only group paths by material for the shading launch; unsorted, every
-    // surface hit goes to the first.
-    uint32_t key        = r.slot == kNone ? kBinMiss : kBinDiffuse + kind;
     if (MEDIA && s.medium_count > 0) {
-        // MediumField::sample over [minimum, hit ? distance : maximum]
-        // (src/render/path_tracer.cpp:170-177).
-        Pcg32  rng   = rng_of(a.st.rng[path]);
-        float4 beta4 = a.st.beta[path];
-        bool   scattered;
-        float  scatter_t = 0, g = 0;
-        const f3 w = field_sample(s, xyz(o4), xyz(d4), o4.w, r.slot != kNone ? r.t : d4.w, rng,
-                                  scattered, scatter_t, g, error);
-        f3 beta = xyz(beta4) * w;
-        a.st.rng[path]  = rng_words(rng);  // not the sector: its shadow ray may be adding radiance
-        a.st.beta[path] = f4(beta, beta4.w);
-        if (!finite3(beta) || beta.x < 0 || beta.y < 0 || beta.z < 0) {
-            error |= kErrorRadiance;
-            key = kNone;
-        } else if (max3(beta) == 0) {
-            key = kNone;
-        } else if (scattered) {
-            a.st.hit[path] = make_float4(scatter_t, g, 0, 0);
-            key            = kBinMedium;
-        }
+        bin = sample_media(a, s, path, o4, d4, t, bin, error);
     }
-    return key;
+    return bin;
 }
 
-// Any hit of one shadow segment; adds the contribution (times the media transmittance) when
-// the segment is clear.
+// After the any-hit test of a shadow segment: adds the contribution (times the media
+// transmittance) when the segment is clear.
+template <bool MEDIA>
+__device__ __forceinline__ void finish_shadow(const KernelArgs& a, const DeviceScene& s, uint32_t path,
+                                              bool occluded) {
+    if (a.occluded_out) {
+        a.occluded_out[path] = occluded ? 1 : 0;
+    }
+    if (!occluded) {
+        f3 c = xyz(a.st.shadow_c[path]);
+        if (MEDIA && s.medium_count > 0) {
+            const float4 o4 = a.st.shadow_o[path];
+            c = c * field_transmittance(s, xyz(o4), xyz(a.st.shadow_d[path]), 0.0f, o4.w);
+        }
+        const float4 L      = a.st.radiance[path];
+        a.st.radiance[path] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0);
+    }
+}
+
+// Any hit of one shadow segment and what follows it.
 template <bool MEDIA, bool TWO>
 __device__ __forceinline__ void shadow_item(const KernelArgs& a, const DeviceScene& s, uint32_t path,
                                             TraceCounters& tc, unsigned& error) {
@@ -316,70 +351,162 @@ __device__ __forceinline__ void shadow_item(const KernelArgs& a, const DeviceSce
     load_pair(a.st.shadow_o, path, o4, d4);
     RayQuery q;
     q.init(xyz(o4), xyz(d4));
-    const TraceResult r = trace_scene<true, TWO>(s, q, 0.0f, o4.w, tc, error);
-    if (a.occluded_out) {
-        a.occluded_out[path] = r.slot != kNone ? 1 : 0;
+    bool occluded;
+    if (TWO && s.two_level) {
+        occluded = trace2<true>(s, q, 0.0f, o4.w, tc, error).slot != kNone;
+    } else {
+        occluded = trace<true>(s, q, 0.0f, o4.w, [&] { return xyz(a.st.shadow_d[path]); }, tc, error).slot !=
+                   kNone;
     }
-    if (r.slot == kNone) {
-        f3 c = xyz(a.st.shadow_c[path]);
-        if (MEDIA && s.medium_count > 0) {
-            c = c * field_transmittance(s, xyz(o4), xyz(d4), 0.0f, o4.w);
-        }
-        const float4 L      = a.st.radiance[path];
-        a.st.radiance[path] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0);
-    }
+    finish_shadow<MEDIA>(a, s, path, occluded);
 }
+
+// Queue items of stream_rays: extension rays (SHADOW = false) or shadow segments of a wave's paths.
+template <bool SHADOW, bool MEDIA, bool BATCH> struct QueueIo {
+    const KernelArgs& a;
+    const uint32_t*   queue;
+    uint32_t*         bins;
+    bool              sorted;
+    unsigned          error = 0;
+    uint32_t          path  = 0;
+    const WaveSegment* g    = nullptr;
+    const float4*     segment_nodes = nullptr;  // of a multi-job wave's lane
+    const float4*     segment_tris  = nullptr;
+
+    __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) {
+        path = queue[i];
+        if constexpr (BATCH) {
+            g             = segment_of<BATCH>(a, path);
+            segment_nodes = g->scene.nodes;
+            segment_tris  = g->scene.tris;
+        }
+        if constexpr (SHADOW) {
+            load_pair(a.st.shadow_o, path, o, d);
+        } else {
+            load_pair(a.st.ray_o, path, o, d);
+        }
+    }
+    __device__ __forceinline__ const DeviceScene& scene() const { return scene_of<BATCH>(a, g); }
+    __device__ __forceinline__ const float4* nodes() const { return BATCH ? segment_nodes : a.scene.nodes; }
+    __device__ __forceinline__ const float4* tris() const { return BATCH ? segment_tris : a.scene.tris; }
+    __device__ __forceinline__ f3 direction() const { return xyz(SHADOW ? a.st.shadow_d[path] : a.st.ray_d[path]); }
+    __device__ __forceinline__ void fail(unsigned bits) { note_error<BATCH>(g, bits, error); }
+    __device__ __forceinline__ void finish(bool done, const StreamRay& ray, const NearestHit& hit) {
+        uint32_t key = kNone;
+        if (done) {
+            if constexpr (SHADOW) {
+                finish_shadow<MEDIA>(a, scene(), path, hit.slot != kNone);
+            } else {
+                key = store_hit(a, scene(), ray.triangle_ray(), path, hit, sorted);
+                if constexpr (MEDIA) {
+                    a.st.bin[path] = key;  // medium_kernel bins the path
+                }
+            }
+        }
+        if constexpr (!SHADOW && !MEDIA) {
+            warp_append(key, path, bins, a.q.bins, a.capacity);
+        }
+    }
+};
 
 // One persistent launch per bounce traverses both queues: the bounce's extension rays first,
 // then the shadow segments the previous bounce's shading queued (their contributions land
-// before this bounce's shading adds emission, the reference's accumulation order). Warps fetch
-// 32 consecutive items, so only the warp at the boundary mixes the two kinds. 8 resident blocks
-// per SM (<= 64 registers): the traversal is latency bound and more warps hide it. In a
-// multi-job wave (BATCH) every path finds its scene through its segment. With two-level scenes
-// in the launch (TWO) the kernel also carries the two-level traversal and runs 5 blocks per SM
-// (<= 102 registers) so that its larger state stays in registers.
+// before this bounce's shading adds emission, the reference's accumulation order). Flattened
+// scenes are streamed (stream.cuh) with 8 resident blocks per SM (<= 64 registers; 7 blocks of 72
+// were 1-3% slower): the traversal waits on loads and more warps hide them. In a multi-job wave
+// (BATCH) every path finds its scene through its segment. With two-level scenes in the launch (TWO)
+// warps fetch 32 items at a time and the kernel carries the two-level traversal; it runs 5 blocks
+// per SM (<= 102 registers) so that its larger state stays in registers.
 template <bool MEDIA, bool BATCH, bool TWO>
-__global__ void __launch_bounds__(128, TWO ? 5 : 8) trace_kernel(KernelArgs a) {
+__global__ void __launch_bounds__(kStreamBlock, TWO ? 5 : 8) trace_kernel(KernelArgs a) {
     BounceCounters* ctr      = a.q.counters + a.bounce;
     const uint32_t  n_ext    = ctr->ext;
     const uint32_t  n_shadow = a.bounce > 0 ? a.q.counters[a.bounce - 1].shadow : 0;
-    const uint32_t  total    = n_ext + n_shadow;
     const bool      sorted   = !BATCH || n_ext >= a.wave->sort_threshold;
     const uint32_t* in       = a.q.ext[a.bounce & 1];
     TraceCounters   tc_ext{0, 0}, tc_shadow{0, 0};
     unsigned        error = 0;
-    const int       lane  = lane_id();
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) {
-            base = atomicAdd(&ctr->work_extend, 32u);
+    if constexpr (!TWO) {
+        extern __shared__ int2 stacks[];
+        if (n_ext) {
+            QueueIo<false, MEDIA, BATCH> io{a, in, ctr->bins, sorted};
+            stream_rays<false>(io, n_ext, &ctr->work_extend, stacks, tc_ext);
+            error |= io.error;
         }
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= total) {
-            break;
+        if (n_shadow) {
+            QueueIo<true, MEDIA, BATCH> io{a, a.q.shadow, nullptr, false};
+            stream_rays<true>(io, n_shadow, &ctr->work_shadow, stacks, tc_shadow);
+            error |= io.error;
         }
-        const uint32_t i    = base + lane;
-        uint32_t       key  = kNone;
-        uint32_t       path = 0;
-        if (i < total) {
-            path                 = i < n_ext ? in[i] : a.q.shadow[i - n_ext];
-            const WaveSegment* g = segment_of<BATCH>(a, path);
-            unsigned           e = 0;
-            if (i < n_ext) {
-                key = extend_item<MEDIA, TWO>(a, scene_of<BATCH>(a, g), path, sorted, tc_ext, e);
-            } else {
-                shadow_item<MEDIA, TWO>(a, scene_of<BATCH>(a, g), path, tc_shadow, e);
+    } else {
+        const uint32_t total = n_ext + n_shadow;
+        const int      lane  = lane_id();
+        while (true) {
+            uint32_t base = 0;
+            if (lane == 0) {
+                base = atomicAdd(&ctr->work_extend, 32u);
             }
-            note_error<BATCH>(g, e, error);
-        }
-        if (base < n_ext) {
-            warp_append(key, path, ctr->bins, a.q.bins, a.capacity);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= total) {
+                break;
+            }
+            const uint32_t i    = base + lane;
+            uint32_t       key  = kNone;
+            uint32_t       path = 0;
+            if (i < total) {
+                path                 = i < n_ext ? in[i] : a.q.shadow[i - n_ext];
+                const WaveSegment* g = segment_of<BATCH>(a, path);
+                unsigned           e = 0;
+                if (i < n_ext) {
+                    key = extend_item<MEDIA, TWO>(a, scene_of<BATCH>(a, g), path, sorted, tc_ext, e);
+                } else {
+                    shadow_item<MEDIA, TWO>(a, scene_of<BATCH>(a, g), path, tc_shadow, e);
+                }
+                note_error<BATCH>(g, e, error);
+            }
+            if (base < n_ext) {
+                warp_append(key, path, ctr->bins, a.q.bins, a.capacity);
+            }
         }
     }
     warp_add_stat(a.q.stats + kStatExtendBounds, tc_ext.bounds);
     warp_add_stat(a.q.stats + kStatExtendTriangles, tc_ext.triangles);
     warp_add_stat(a.q.stats + kStatShadowBounds, tc_shadow.bounds);
     warp_add_stat(a.q.stats + kStatShadowTriangles, tc_shadow.triangles);
+    if (error) {
+        atomicOr(a.q.error, error);
+    }
+}
+
+// Waves with media (flattened scenes), after the traversal launch: the free-flight sample of every
+// extension ray over its hit interval, then its bin. A launch of its own because its registers and
+// its latency (path records, transcendentals) are not the traversal's: inside the streamed kernel,
+// at each refill, it made the traversal of a fogged 1M-triangle frame 24.9 ms against 14.3 ms for
+// the two launches together (and 16.1 ms before streaming).
+template <bool BATCH> __global__ void __launch_bounds__(128) medium_kernel(KernelArgs a) {
+    BounceCounters* ctr   = a.q.counters + a.bounce;
+    const uint32_t  n     = ctr->ext;
+    const uint32_t* in    = a.q.ext[a.bounce & 1];
+    unsigned        error = 0;
+    const uint32_t  step  = gridDim.x * blockDim.x;
+    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += step) {
+        const uint32_t i   = base + lane_id();
+        uint32_t       bin = kNone, path = 0;
+        if (i < n) {
+            path                 = in[i];
+            const WaveSegment* g = segment_of<BATCH>(a, path);
+            const DeviceScene& s = scene_of<BATCH>(a, g);
+            bin                  = a.st.bin[path];
+            if (s.medium_count > 0) {
+                float4   o4, d4;
+                unsigned e = 0;
+                load_pair(a.st.ray_o, path, o4, d4);
+                bin = sample_media(a, s, path, o4, d4, bin == kBinMiss ? d4.w : a.st.hit[path].x, bin, e);
+                note_error<BATCH>(g, e, error);
+            }
+        }
+        warp_append(bin, path, ctr->bins, a.q.bins, a.capacity);
+    }
     if (error) {
         atomicOr(a.q.error, error);
     }
@@ -1000,9 +1127,9 @@ LaunchShape& launch_shape() {
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current);
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_kernel<false, false, false>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_kernel<false, false, false>, kStreamBlock, kStreamSharedBytes);
         shape.trace_blocks[0] = sms * std::max(1, per);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_kernel<true, false, false>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_kernel<true, false, false>, kStreamBlock, kStreamSharedBytes);
         shape.trace_blocks[1] = sms * std::max(1, per);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_kernel<false, false, true>, 128, 0);
         shape.trace_blocks[2] = sms * std::max(1, per);
@@ -1259,7 +1386,7 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
     KernelTiming&      timing = kernel_timing();
     bool               timed  = false;
     timed = timing.enabled.load();
-    note_launches(1 + 2ull * (params.maximum_depth + 1) + (ray_sort ? 4ull * params.maximum_depth : 0ull) +
+    note_launches(1 + (media && !two ? 3ull : 2ull) * (params.maximum_depth + 1) + (ray_sort ? 4ull * params.maximum_depth : 0ull) +
                   (init.capture ? 1 : 0));
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
     // The timed launches are the trace kernels: nearest-hit and shadow tests both count.
@@ -1280,8 +1407,8 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
         // The first shadow rays (queued by bounce 0's shading) are traced with bounce 1.
         a.occluded_out = bounce == 1 && init.capture ? init.capture->occluded : nullptr;
         switch (variant) {
-        case 0: trace_kernel<false, false, false><<<shape.trace_blocks[0], 128, 0, stream>>>(a); break;
-        case 1: trace_kernel<true, false, false><<<shape.trace_blocks[1], 128, 0, stream>>>(a); break;
+        case 0: trace_kernel<false, false, false><<<shape.trace_blocks[0], kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
+        case 1: trace_kernel<true, false, false><<<shape.trace_blocks[1], kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 2: trace_kernel<false, false, true><<<shape.trace_blocks[2], 128, 0, stream>>>(a); break;
         default: trace_kernel<true, false, true><<<shape.trace_blocks[3], 128, 0, stream>>>(a); break;
         }
@@ -1289,6 +1416,9 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
         if (timed) {
             cudaEventRecord(e1, stream);
             events.emplace_back(e0, e1);
+        }
+        if (media && !two) {
+            medium_kernel<false><<<shape.shade_blocks, 128, 0, stream>>>(a);
         }
         if (two) {
             shade_kernel<false, true><<<shape.shade_blocks_two, 128, 0, stream>>>(a);
@@ -1329,8 +1459,8 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
 void Engine::batch_occupancy(int& trace_blocks_per_sm, int& shade_blocks_per_sm) {
     int a = 0, b = 0, c = 0;
     int f = 0;
-    MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, trace_kernel<false, true, false>, 128, 0));
-    MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_kernel<true, true, false>, 128, 0));
+    MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, trace_kernel<false, true, false>, kStreamBlock, kStreamSharedBytes));
+    MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_kernel<true, true, false>, kStreamBlock, kStreamSharedBytes));
     MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, shade_kernel<true, false>, 128, 0));
     MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, shade_kernel<true, true>, 128, 0));
     trace_blocks_per_sm = std::max(1, std::min(a, b));
@@ -1370,10 +1500,13 @@ void Engine::enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, b
     for (uint32_t bounce = 0; bounce <= maximum_depth; ++bounce) {
         a.bounce = bounce;
         switch ((media ? 1 : 0) + (two ? 2 : 0)) {
-        case 0: trace_kernel<false, true, false><<<shape.trace_blocks, 128, 0, stream>>>(a); break;
-        case 1: trace_kernel<true, true, false><<<shape.trace_blocks, 128, 0, stream>>>(a); break;
+        case 0: trace_kernel<false, true, false><<<shape.trace_blocks, kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
+        case 1: trace_kernel<true, true, false><<<shape.trace_blocks, kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 2: trace_kernel<false, true, true><<<trace_blocks, 128, 0, stream>>>(a); break;
         default: trace_kernel<true, true, true><<<trace_blocks, 128, 0, stream>>>(a); break;
+        }
+        if (media && !two) {
+            medium_kernel<true><<<shape.shade_blocks, 128, 0, stream>>>(a);
         }
         if (two) {
             shade_kernel<true, true><<<shape.shade_blocks, 128, 0, stream>>>(a);
@@ -1586,3 +1719,11 @@ void copy_path_radiance(Workspace& ws, uint32_t count, float* device_out, cudaSt
 }
 
 }  // namespace mr
+
+#ifdef X_STAT
+extern "C" void x_stat(unsigned long long* out) {
+    cudaMemcpyFromSymbol(out, mr::g_stat, 16 * 8);
+    unsigned long long z[16] = {};
+    cudaMemcpyToSymbol(mr::g_stat, z, 16 * 8);
+}
+#endif

@@ -24,8 +24,9 @@ struct BounceCounters {
     uint32_t ext;                 // paths entering this bounce
     uint32_t bins[kBinCount];
     uint32_t shadow;
-    uint32_t work_extend;  // work fetch of the bounce's trace launch
-    uint32_t pad[7];
+    uint32_t work_extend;  // work fetch of the bounce's trace launch: extension rays (two-level: both kinds)
+    uint32_t work_shadow;  // and shadow rays
+    uint32_t pad[6];
 };
 
 enum Stat : int {
@@ -113,7 +114,7 @@ __device__ __forceinline__ void store_pair(const RecordField<float4, STRIDE>& lo
 // record per path slot. Kernels reach paths by slot in queue and bin order, which scatters the
 // slots; a record keeps what one kernel reads of a path in whole 32-byte sectors instead of a
 // 16-byte piece of a sector in each of a dozen arrays. Path record sectors: the ray (ray_o,
-// ray_d: what traversal reads), the hit (hit, hit_slot, segment: what traversal writes),
+// ray_d: what traversal reads), the hit (hit, hit_slot, segment, bin: what traversal writes),
 // throughput and previous vertex (beta, prev), radiance and RNG (radiance, rng). Shading reads
 // the four and writes all but the hit, one 32-byte access per sector; a shadow test reads the shadow record's ray and, when the segment is clear,
 // its contribution and the path's radiance sector.
@@ -134,6 +135,7 @@ struct PathState {
     PathField<float4>     hit;       // distance, barycentrics (medium: distance, g)    (+32)
     PathField<uint32_t>   hit_slot;  // triangle slot, kNone on a miss                  (+48)
     PathField<uint32_t>   segment;   // multi-job waves: the path's wave segment        (+56)
+    PathField<uint32_t>   bin;       // streamed waves with media: the hit's bin        (+60)
     PathField<float4>     beta;      // throughput, eta scale                           (+64)
     PathField<float4>     prev;      // previous scattering vertex and its pdf, kDeltaPdf
                                      // where that was a delta event or the camera     (+80)
@@ -151,6 +153,7 @@ struct PathState {
         hit.base      = paths + 32;
         hit_slot.base = paths + 48;
         segment.base  = with_segment ? paths + 56 : nullptr;
+        bin.base      = paths + 60;
         beta.base     = paths + 64;
         prev.base     = paths + 80;
         radiance.base = paths + 96;
@@ -264,8 +267,8 @@ class Engine {
     static void batch_occupancy(int& trace_blocks_per_sm, int& shade_blocks_per_sm);
 
     // Kernel launches of one wave (paths + resolve).
-    static uint64_t batch_wave_launches(uint32_t maximum_depth, bool ray_sort) {
-        return 2ull + 2ull * (maximum_depth + 1) + (ray_sort ? 4ull * maximum_depth : 0ull);
+    static uint64_t batch_wave_launches(uint32_t maximum_depth, bool media, bool two, bool ray_sort) {
+        return 2ull + (media && !two ? 3ull : 2ull) * (maximum_depth + 1) + (ray_sort ? 4ull * maximum_depth : 0ull);
     }
 };
 

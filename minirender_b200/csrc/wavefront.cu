@@ -1719,11 +1719,3 @@ void copy_path_radiance(Workspace& ws, uint32_t count, float* device_out, cudaSt
 }
 
 }  // namespace mr
-
-#ifdef X_STAT
-extern "C" void x_stat(unsigned long long* out) {
-    cudaMemcpyFromSymbol(out, mr::g_stat, 16 * 8);
-    unsigned long long z[16] = {};
-    cudaMemcpyToSymbol(mr::g_stat, z, 16 * 8);
-}
-#endif

@@ -400,6 +400,24 @@ mr_status mr_intersect(const mr_scene* scene, const mr_ray* rays, size_t count, 
 mr_status mr_occluded(const mr_scene* scene, const mr_ray* rays, size_t count, uint8_t* occluded,
                       mr_trace_statistics* statistics);
 
+/* Rays as separate arrays, for callers that hold them so: 3 floats per ray of `origins` and of
+ * `directions`, and interval ends, one per ray or (count 1) one for all. mr_intersect_arrays and
+ * mr_occluded_arrays are mr_intersect and mr_occluded without packing them first. No reference
+ * counterpart. */
+typedef struct mr_ray_arrays {
+    const float* origins;
+    const float* directions;
+    const float* minimum;
+    const float* maximum;
+    size_t       minimum_count;
+    size_t       maximum_count;
+} mr_ray_arrays;
+
+mr_status mr_intersect_arrays(const mr_scene* scene, const mr_ray_arrays* rays, size_t count, mr_hit* hits,
+                              mr_trace_statistics* statistics);
+mr_status mr_occluded_arrays(const mr_scene* scene, const mr_ray_arrays* rays, size_t count,
+                             uint8_t* occluded, mr_trace_statistics* statistics);
+
 /* PathTracer::trace (src/render/path_tracer.cpp:153-366) for `count` independent paths. The
  * sampler of path i is Sampler::for_sample(keys[3i], keys[3i+1], keys[3i+2])
  * (src/core/sampling.cpp:43-46); rays[i] carries the primary interval. */

@@ -160,6 +160,12 @@ class Ray(C.Structure):
                 ("maximum", C.c_float)]
 
 
+class RayArrays(C.Structure):
+    _fields_ = [("origins", C.POINTER(C.c_float)), ("directions", C.POINTER(C.c_float)),
+                ("minimum", C.POINTER(C.c_float)), ("maximum", C.POINTER(C.c_float)),
+                ("minimum_count", C.c_size_t), ("maximum_count", C.c_size_t)]
+
+
 class Hit(C.Structure):
     _fields_ = [("distance", C.c_float), ("instance_index", C.c_uint32),
                 ("triangle_index", C.c_uint32), ("primitive", C.c_uint32),
@@ -238,6 +244,8 @@ SIGNATURES = {
     "mr_scene_build_seconds": (C.c_int, [VP, P(C.c_double)]),
     "mr_intersect": (C.c_int, [VP, P(Ray), C.c_size_t, P(Hit), P(TraceStatistics)]),
     "mr_occluded": (C.c_int, [VP, P(Ray), C.c_size_t, P(C.c_uint8), P(TraceStatistics)]),
+    "mr_intersect_arrays": (C.c_int, [VP, P(RayArrays), C.c_size_t, P(Hit), P(TraceStatistics)]),
+    "mr_occluded_arrays": (C.c_int, [VP, P(RayArrays), C.c_size_t, P(C.c_uint8), P(TraceStatistics)]),
     "mr_trace_paths": (C.c_int, [VP, P(IntegratorSettings), P(Ray), P(C.c_uint64), C.c_size_t,
                                  P(C.c_float), P(PathStatistics)]),
     "mr_sample_pixels": (C.c_int, [VP, P(IntegratorSettings), P(RenderSettings),

@@ -75,12 +75,34 @@ def pack_rays(origins, directions, minimum, maximum) -> np.ndarray:
     """Packs rays into mr_ray records (8 float32 each)."""
     o = _f32(origins, (-1, 3))
     n = o.shape[0]
-    rays = np.zeros((n, 8), np.float32)
+    rays = np.empty((n, 8), np.float32)
     rays[:, 0:3] = o
     rays[:, 3:6] = _f32(directions, (-1, 3))
     rays[:, 6] = np.broadcast_to(np.asarray(minimum, np.float32), (n,))
     rays[:, 7] = np.broadcast_to(np.asarray(maximum, np.float32), (n,))
     return rays
+
+
+def ray_arrays(origins, directions, minimum, maximum):
+    """The same rays as mr_ray_arrays over the caller's own memory where it is contiguous float32.
+    Returns the record, the ray count and the arrays it points into."""
+    o, d = _f32(origins, (-1, 3)), _f32(directions, (-1, 3))
+    n = o.shape[0]
+    if d.shape[0] != n:
+        d = np.ascontiguousarray(np.broadcast_to(d, (n, 3)))
+    ends = []
+    for end in (minimum, maximum):
+        end = np.asarray(end, np.float32)
+        ends.append(np.ascontiguousarray(end.reshape(1) if end.size == 1 and end.ndim <= 1
+                                         else np.broadcast_to(end, (n,))))
+    record = _abi.RayArrays(_ptr(o, C.c_float), _ptr(d, C.c_float), _ptr(ends[0], C.c_float),
+                            _ptr(ends[1], C.c_float), ends[0].size, ends[1].size)
+    return record, n, (o, d, *ends)
+
+
+# mr_hit as a numpy record.
+HIT_DTYPE = np.dtype([("distance", "<f4"), ("instance", "<u4"), ("triangle", "<u4"), ("primitive", "<u4"),
+                      ("barycentric", "<f4", 3), ("front_face", "<u4")])
 
 
 class Scene:
@@ -167,27 +189,22 @@ class Scene:
     # ---- SceneBvh queries (src/render/bvh.cpp:372-384) ----
 
     def intersect(self, origins, directions, minimum=1e-5, maximum=np.inf):
-        rays = pack_rays(origins, directions, minimum, maximum)
-        n = rays.shape[0]
-        hits = (_abi.Hit * max(1, n))()
+        rays, n, _keep = ray_arrays(origins, directions, minimum, maximum)
+        raw = np.empty(n, HIT_DTYPE)  # every record is written by the query
         stats = _abi.TraceStatistics()
-        check(self.lib.mr_intersect(self.handle, C.cast(rays.ctypes.data, C.POINTER(_abi.Ray)), n,
-                                    hits, C.byref(stats)), self.lib)
-        raw = np.frombuffer(hits, dtype=np.dtype([("distance", "<f4"), ("instance", "<u4"),
-                                                  ("triangle", "<u4"), ("primitive", "<u4"),
-                                                  ("barycentric", "<f4", 3),
-                                                  ("front_face", "<u4")]))[:n].copy()
+        check(self.lib.mr_intersect_arrays(self.handle, C.byref(rays), n,
+                                           C.cast(raw.ctypes.data, C.POINTER(_abi.Hit)),
+                                           C.byref(stats)), self.lib)
         return raw, {"bounds_tests": stats.bounds_tests, "triangle_tests": stats.triangle_tests}
 
     def occluded(self, origins, directions, minimum=1e-5, maximum=np.inf):
-        rays = pack_rays(origins, directions, minimum, maximum)
-        n = rays.shape[0]
-        out = np.zeros(max(1, n), np.uint8)
+        rays, n, _keep = ray_arrays(origins, directions, minimum, maximum)
+        out = np.empty(n, np.uint8)
         stats = _abi.TraceStatistics()
-        check(self.lib.mr_occluded(self.handle, C.cast(rays.ctypes.data, C.POINTER(_abi.Ray)), n,
-                                   _ptr(out, C.c_uint8), C.byref(stats)), self.lib)
-        return out[:n].astype(bool), {"bounds_tests": stats.bounds_tests,
-                                      "triangle_tests": stats.triangle_tests}
+        check(self.lib.mr_occluded_arrays(self.handle, C.byref(rays), n, _ptr(out, C.c_uint8),
+                                          C.byref(stats)), self.lib)
+        return out.view(bool), {"bounds_tests": stats.bounds_tests,
+                                "triangle_tests": stats.triangle_tests}
 
 
 class PathTracer:

@@ -59,15 +59,6 @@ void copy_path_radiance(Workspace& ws, uint32_t count, float* device_out, cudaSt
 
 namespace {
 
-// A non-blocking stream owned by one API call.
-struct CallStream {
-    cudaStream_t stream = nullptr;
-    CallStream() { MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
-    ~CallStream() { cudaStreamDestroy(stream); }
-    CallStream(const CallStream&)            = delete;
-    CallStream& operator=(const CallStream&) = delete;
-};
-
 thread_local std::string last_error;
 
 template <typename F> mr_status guarded(F&& f) {
@@ -85,6 +76,13 @@ template <typename F> mr_status guarded(F&& f) {
         return MR_RUNTIME_ERROR;
     }
 }
+
+// Counters and flags of a ray query, copied back at once.
+struct QueryStatus {
+    unsigned long long bounds, triangles;
+    unsigned           error;    // ErrorBits
+    unsigned           invalid;  // a ray that validate_ray refuses
+};
 
 // RayQuery constructor and RayInterval::validate (src/render/intersection.cpp:22-26,52-61).
 void validate_ray(const mr_ray& r) {
@@ -114,18 +112,68 @@ template <typename T> DeviceBuffer<T> upload(const T* host, size_t count, cudaSt
     return b;
 }
 
-__global__ void query_kernel(DeviceScene s, const mr_ray* rays, size_t count, int any_hit,
-                             mr_hit* hits, uint8_t* occluded, unsigned long long* counters,
-                             unsigned* error) {
+// validate_ray on the device: the squared length in FP64 with the host check's operation order, so
+// it refuses exactly the rays the host refuses; no traversal arithmetic uses FP64.
+__device__ __forceinline__ bool valid_ray(const mr_ray& r) {
+    bool ok = true;
+    for (int a = 0; a < 3; ++a) {
+        ok = ok && isfinite(r.origin[a]) && isfinite(r.direction[a]);
+    }
+    const double x = r.direction[0], y = r.direction[1], z = r.direction[2];
+    const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+    return ok && fabs(d2 - 1.0) <= 1e-4 && isfinite(r.minimum) && r.minimum >= 0 && !isnan(r.maximum) &&
+           r.maximum >= r.minimum;
+}
+
+// Rays of a query, in one array of records or in separate arrays: element i of each field is
+// `step` floats after element i - 1.
+struct QueryRays {
+    const float *origin, *direction, *minimum, *maximum;
+    uint32_t     origin_step, direction_step, minimum_step, maximum_step;
+    MR_HD mr_ray operator[](size_t i) const {
+        const float* o = origin + i * origin_step;
+        const float* d = direction + i * direction_step;
+        return {{o[0], o[1], o[2]}, {d[0], d[1], d[2]}, minimum[i * minimum_step], maximum[i * maximum_step]};
+    }
+};
+
+QueryRays records(const mr_ray* rays) {
+    static_assert(sizeof(mr_ray) == 8 * sizeof(float), "mr_ray is eight floats");
+    const float* f = reinterpret_cast<const float*>(rays);
+    return {f, f + 3, f + 6, f + 7, 8, 8, 8, 8};
+}
+
+QueryRays arrays(const mr_ray_arrays* rays, size_t count) {
+    require(rays != nullptr, "Ray arrays are null");
+    require((rays->minimum_count == 1 || rays->minimum_count == count) &&
+                (rays->maximum_count == 1 || rays->maximum_count == count),
+            "Interval ends are one per ray or one for all");
+    return {rays->origins, rays->directions, rays->minimum, rays->maximum, 3, 3,
+            rays->minimum_count == 1 ? 0u : 1u, rays->maximum_count == 1 ? 0u : 1u};
+}
+
+__global__ void query_kernel(DeviceScene s, QueryRays rays, size_t count, int any_hit,
+                             mr_hit* hits, uint8_t* occluded, QueryStatus* status) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     TraceCounters tc{0, 0};
     unsigned      err = 0;
-    if (i < count) {
-        const mr_ray r = rays[i];
-        RayQuery     q;
+    bool          valid = i < count;
+    mr_ray        r{};
+    if (valid) {
+        r     = rays[i];
+        valid = valid_ray(r);
+        if (!valid) {
+            status->invalid = 1;
+        }
+    }
+    if (valid) {
+        RayQuery q;
         q.init(make(r.origin[0], r.origin[1], r.origin[2]),
                make(r.direction[0], r.direction[1], r.direction[2]));
-        const auto direction = [&] { return make(rays[i].direction[0], rays[i].direction[1], rays[i].direction[2]); };
+        const auto direction = [&] {
+            const mr_ray again = rays[i];
+            return make(again.direction[0], again.direction[1], again.direction[2]);
+        };
         if (any_hit) {
             const uint32_t slot =
                 s.two_level ? trace2<true>(s, q, r.minimum, r.maximum, tc, err).slot
@@ -164,56 +212,76 @@ __global__ void query_kernel(DeviceScene s, const mr_ray* rays, size_t count, in
     const uint32_t b = __reduce_add_sync(0xffffffffu, tc.bounds);
     const uint32_t t = __reduce_add_sync(0xffffffffu, tc.triangles);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(counters, static_cast<unsigned long long>(b));
-        atomicAdd(counters + 1, static_cast<unsigned long long>(t));
+        atomicAdd(&status->bounds, static_cast<unsigned long long>(b));
+        atomicAdd(&status->triangles, static_cast<unsigned long long>(t));
     }
     if (err) {
-        atomicOr(error, err);
+        atomicOr(&status->error, err);
     }
 }
 
-void run_query(const Scene& scene, const mr_ray* rays, size_t count, int any_hit, mr_hit* hits,
+// `packed`: the rays are records starting at `rays.origin`.
+void run_query(const Scene& scene, const QueryRays& rays, bool packed, size_t count, int any_hit, mr_hit* hits,
                uint8_t* occluded, mr_trace_statistics* statistics) {
-    require(rays != nullptr || count == 0, "Ray buffer is null");
+    require((rays.origin && rays.direction && rays.minimum && rays.maximum) || count == 0, "Ray buffer is null");
     require((any_hit ? occluded != nullptr : hits != nullptr) || count == 0, "Output buffer is null");
-    for (size_t i = 0; i < count; ++i) {
-        validate_ray(rays[i]);
-    }
-    cudaStream_t stream = nullptr;
-    auto         d_rays = upload(rays, count, stream);
-    DeviceBuffer<mr_hit>             d_hits;
-    DeviceBuffer<uint8_t>            d_occ;
-    DeviceBuffer<unsigned long long> d_counters;
-    DeviceBuffer<unsigned>           d_error;
-    d_hits.allocate(any_hit ? 1 : std::max<size_t>(1, count));
-    d_occ.allocate(any_hit ? std::max<size_t>(1, count) : 1);
-    d_counters.allocate(2);
-    d_error.allocate(1);
-    MR_CUDA(cudaMemsetAsync(d_counters.ptr, 0, 2 * sizeof(unsigned long long), stream));
-    MR_CUDA(cudaMemsetAsync(d_error.ptr, 0, sizeof(unsigned), stream));
+    // The call's own stream and stream-ordered buffers: no device-wide wait from an allocation.
+    CallStream                call;
+    AllocationScope           scope(call.stream);
+    const cudaStream_t        stream = call.stream;
+    DeviceBuffer<mr_hit>      d_hits;
+    DeviceBuffer<uint8_t>     d_occ;
+    DeviceBuffer<QueryStatus> d_status;
+    QueryStatus               result{};
+    d_status.allocate(1);
+    MR_CUDA(cudaMemsetAsync(d_status.ptr, 0, sizeof(QueryStatus), stream));
     if (count) {
+        DeviceBuffer<float> fields[4];
+        QueryRays           device = rays;
+        if (packed) {
+            fields[0] = upload(rays.origin, 8 * count, stream);
+            device    = records(reinterpret_cast<const mr_ray*>(fields[0].ptr));
+        } else {
+            fields[0] = upload(rays.origin, 3 * count, stream);
+            fields[1] = upload(rays.direction, 3 * count, stream);
+            fields[2] = upload(rays.minimum, rays.minimum_step ? count : 1, stream);
+            fields[3] = upload(rays.maximum, rays.maximum_step ? count : 1, stream);
+            device.origin    = fields[0].ptr;
+            device.direction = fields[1].ptr;
+            device.minimum   = fields[2].ptr;
+            device.maximum   = fields[3].ptr;
+        }
+        if (any_hit) {
+            d_occ.allocate(count);
+        } else {
+            d_hits.allocate(count);
+        }
         query_kernel<<<static_cast<unsigned>((count + 127) / 128), 128, 0, stream>>>(
-            scene.d, d_rays.ptr, count, any_hit, d_hits.ptr, d_occ.ptr, d_counters.ptr, d_error.ptr);
+            scene.d, device, count, any_hit, d_hits.ptr, d_occ.ptr, d_status.ptr);
         MR_CUDA(cudaGetLastError());
+        MR_CUDA(cudaMemcpyAsync(&result, d_status.ptr, sizeof(result), cudaMemcpyDeviceToHost, stream));
+        MR_CUDA(cudaStreamSynchronize(stream));
+        if (result.invalid) {  // refused by the device's check: the host's names the fault
+            for (size_t i = 0; i < count; ++i) {
+                validate_ray(rays[i]);
+            }
+            fail(MR_INVALID_ARGUMENT, "Ray is invalid");
+        }
         if (any_hit) {
             MR_CUDA(cudaMemcpyAsync(occluded, d_occ.ptr, count, cudaMemcpyDeviceToHost, stream));
         } else {
             MR_CUDA(cudaMemcpyAsync(hits, d_hits.ptr, count * sizeof(mr_hit), cudaMemcpyDeviceToHost, stream));
         }
+        MR_CUDA(cudaStreamSynchronize(stream));
     }
-    unsigned long long counters[2] = {0, 0};
-    unsigned           error       = 0;
-    MR_CUDA(cudaMemcpyAsync(counters, d_counters.ptr, sizeof(counters), cudaMemcpyDeviceToHost, stream));
-    MR_CUDA(cudaMemcpyAsync(&error, d_error.ptr, sizeof(error), cudaMemcpyDeviceToHost, stream));
-    MR_CUDA(cudaStreamSynchronize(stream));
     std::string message;
-    const mr_status status = error_status(error, message);
+    const mr_status status = error_status(result.error, message);
     if (status != MR_OK) {
         fail(status, message);
     }
     if (statistics) {
-        statistics->bounds_tests += counters[0];
-        statistics->triangle_tests += counters[1];
+        statistics->bounds_tests += result.bounds;
+        statistics->triangle_tests += result.triangles;
     }
 }
 
@@ -223,7 +291,9 @@ void run_paths(const Scene& scene, const IntegratorParams& params, WaveInit init
                const uint64_t* samples, float* radiance, mr_ray* camera_rays,
                mr_path_statistics* statistics, mr_ray* shadow_rays = nullptr,
                uint8_t* has_shadow = nullptr, uint8_t* occluded = nullptr) {
-    cudaStream_t stream = nullptr;
+    CallStream         call;
+    AllocationScope    scope(call.stream);
+    const cudaStream_t stream = call.stream;
     const size_t chunk  = std::min<size_t>(std::max<size_t>(1, count), size_t(1) << 22);
     auto         ws     = acquire_workspace(chunk, params.maximum_depth + 1, 1);
     reset_statistics(*ws, stream);
@@ -357,8 +427,9 @@ void session_run(mr_session* s, const Scene* scene, IntegratorParams params, mr_
                  mr_session_settings settings) {
     try {
         MR_CUDA(cudaSetDevice(s->device));
-        cudaStream_t stream;
-        MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        CallStream         call;
+        AllocationScope    scope(call.stream);
+        const cudaStream_t stream = call.stream;
         const size_t pixels = static_cast<size_t>(render.width) * render.height;
         const size_t capacity =
             std::min<size_t>(pixels * std::min<uint32_t>(render.samples_per_pixel, settings.batch_samples),
@@ -416,7 +487,6 @@ void session_run(mr_session* s, const Scene* scene, IntegratorParams params, mr_
             s->statistics = stats;
         }
         release_workspace(ws);
-        cudaStreamDestroy(stream);
         if (cancelled) {
             std::lock_guard<std::mutex> lock(s->control);
             s->state    = MR_STATE_CANCELLED;
@@ -604,12 +674,36 @@ mr_status mr_scene_build_seconds(const mr_scene* scene, double* seconds) {
 
 mr_status mr_intersect(const mr_scene* scene, const mr_ray* rays, size_t count, mr_hit* hits,
                        mr_trace_statistics* statistics) {
-    return guarded([&] { run_query(scene_of(scene), rays, count, 0, hits, nullptr, statistics); });
+    return guarded([&] {
+        const Scene& s = scene_of(scene);
+        require(rays != nullptr || count == 0, "Ray buffer is null");
+        run_query(s, records(rays), true, count, 0, hits, nullptr, statistics);
+    });
 }
 
 mr_status mr_occluded(const mr_scene* scene, const mr_ray* rays, size_t count, uint8_t* occluded,
                       mr_trace_statistics* statistics) {
-    return guarded([&] { run_query(scene_of(scene), rays, count, 1, nullptr, occluded, statistics); });
+    return guarded([&] {
+        const Scene& s = scene_of(scene);
+        require(rays != nullptr || count == 0, "Ray buffer is null");
+        run_query(s, records(rays), true, count, 1, nullptr, occluded, statistics);
+    });
+}
+
+mr_status mr_intersect_arrays(const mr_scene* scene, const mr_ray_arrays* rays, size_t count, mr_hit* hits,
+                              mr_trace_statistics* statistics) {
+    return guarded([&] {
+        const Scene& s = scene_of(scene);
+        run_query(s, arrays(rays, count), false, count, 0, hits, nullptr, statistics);
+    });
+}
+
+mr_status mr_occluded_arrays(const mr_scene* scene, const mr_ray_arrays* rays, size_t count, uint8_t* occluded,
+                             mr_trace_statistics* statistics) {
+    return guarded([&] {
+        const Scene& s = scene_of(scene);
+        run_query(s, arrays(rays, count), false, count, 1, nullptr, occluded, statistics);
+    });
 }
 
 mr_status mr_trace_paths(const mr_scene* scene, const mr_integrator_settings* integrator,

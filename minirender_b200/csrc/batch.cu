@@ -272,8 +272,9 @@ class Server {
         cudaStreamDestroy(copy_stream_);
     }
 
-    uint64_t submit(const Scene* scene, const mr_render_settings* render,
-                    const mr_integrator_settings* integrator, float* output, bool copy_back = true) {
+    // A validated job, not yet submitted.
+    std::unique_ptr<Job> prepare(const Scene* scene, const mr_render_settings* render,
+                                 const mr_integrator_settings* integrator, float* output, bool copy_back) {
         require(scene != nullptr, "Scene handle is null");
         const IntegratorParams p = integrator_params(integrator);
         validate_render(render);
@@ -295,16 +296,34 @@ class Server {
         if (job->device_bytes > settings_.hbm_budget_bytes) {
             fail(MR_OUT_OF_MEMORY, "The job's buffers exceed the server's HBM budget");
         }
+        return job;
+    }
+
+    uint64_t submit(const Scene* scene, const mr_render_settings* render,
+                    const mr_integrator_settings* integrator, float* output, bool copy_back = true) {
+        std::vector<std::unique_ptr<Job>> one;
+        one.push_back(prepare(scene, render, integrator, output, copy_back));
+        return submit_all(std::move(one)).front();
+    }
+
+    // Submits the jobs together: the controller sees all of them when it packs the next wave. One at
+    // a time, it packed a wave of the first few it happened to see, of a depth that needed a graph of
+    // its own (24 preview jobs: 7 ms, or 20 ms when it did).
+    std::vector<uint64_t> submit_all(std::vector<std::unique_ptr<Job>> jobs) {
+        std::vector<uint64_t>       ids;
         std::lock_guard<std::mutex> lock(mutex_);
         require(!stop_, "The server is shutting down");
-        job->id        = ++last_id_;
-        job->submitted = now();
-        Job* raw       = job.get();
-        jobs_.emplace(raw->id, std::move(job));
-        queued_.push_back(raw);
-        ++stats_.submitted;
+        for (auto& job : jobs) {
+            job->id        = ++last_id_;
+            job->submitted = now();
+            Job* raw       = job.get();
+            jobs_.emplace(raw->id, std::move(job));
+            queued_.push_back(raw);
+            ++stats_.submitted;
+            ids.push_back(raw->id);
+        }
         work_.notify_all();
-        return raw->id;
+        return ids;
     }
 
     bool pause(uint64_t id) {
@@ -1054,10 +1073,13 @@ mr_status run_batch(mr_batch_job* jobs, size_t count, const mr_batch_settings* s
     server.record_after_lanes(marks[0]);
     std::vector<uint64_t> ids(count, 0);
     mr_status first = MR_OK;
+    std::vector<std::unique_ptr<Job>> prepared;
+    std::vector<size_t>               index;
     for (size_t i = 0; i < count; ++i) {
         try {
-            ids[i] = server.submit(scene_ptr(jobs[i].scene), &jobs[i].render, &jobs[i].integrator,
-                                   copy_images ? jobs[i].rgb : nullptr, copy_images && jobs[i].rgb);
+            prepared.push_back(server.prepare(scene_ptr(jobs[i].scene), &jobs[i].render, &jobs[i].integrator,
+                                              copy_images ? jobs[i].rgb : nullptr, copy_images && jobs[i].rgb));
+            index.push_back(i);
         } catch (const Error& e) {
             jobs[i].status = e.status;
             if (first == MR_OK) {
@@ -1065,6 +1087,10 @@ mr_status run_batch(mr_batch_job* jobs, size_t count, const mr_batch_settings* s
                 set_last_error(e.what());
             }
         }
+    }
+    const std::vector<uint64_t> submitted = server.submit_all(std::move(prepared));
+    for (size_t k = 0; k < submitted.size(); ++k) {
+        ids[index[k]] = submitted[k];
     }
     server.wait_all();
     const double seconds = std::chrono::duration<double>(Clock::now() - t0).count();

@@ -641,11 +641,7 @@ void update_mesh(Scene& scene, uint32_t mesh, const float* positions, uint32_t p
     for (uint64_t k = 0; k < 3ull * position_count; ++k) {
         require(std::isfinite(positions[k]), "Mesh position must be finite");
     }
-    struct OwnedStream {
-        cudaStream_t stream = nullptr;
-        OwnedStream() { MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
-        ~OwnedStream() { cudaStreamDestroy(stream); }
-    } owned;
+    CallStream      owned;
     cudaStream_t    stream = owned.stream;
     AllocationScope scope(stream);
     // The new positions pass MeshData::validate's degenerate-triangle check before anything
@@ -685,11 +681,7 @@ void update_mesh(Scene& scene, uint32_t mesh, const float* positions, uint32_t p
 }
 
 void rebuild_after_refit(Scene& scene) {
-    struct OwnedStream {
-        cudaStream_t stream = nullptr;
-        OwnedStream() { MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
-        ~OwnedStream() { cudaStreamDestroy(stream); }
-    } owned;
+    CallStream      owned;
     cudaStream_t    stream = owned.stream;
     AllocationScope scope(stream);
     build_instance_tree(scene, stream);

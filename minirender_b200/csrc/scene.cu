@@ -553,6 +553,51 @@ cudaMemPool_t library_pool() {
     return pools[device];
 }
 
+namespace {
+
+struct PooledStream {
+    int          device;
+    cudaStream_t stream;
+};
+// Never destroyed: streams must not be destroyed after the CUDA runtime at process exit.
+std::mutex& stream_mutex() {
+    static auto* m = new std::mutex;
+    return *m;
+}
+std::vector<PooledStream>& stream_pool() {
+    static auto* streams = new std::vector<PooledStream>;
+    return *streams;
+}
+
+}  // namespace
+
+CallStream::CallStream() {
+    MR_CUDA(cudaGetDevice(&device));
+    {
+        std::lock_guard<std::mutex> lock(stream_mutex());
+        auto& streams = stream_pool();
+        for (size_t i = streams.size(); i > 0; --i) {
+            if (streams[i - 1].device == device) {
+                stream = streams[i - 1].stream;
+                streams.erase(streams.begin() + static_cast<long>(i - 1));
+                return;
+            }
+        }
+    }
+    MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+}
+
+CallStream::~CallStream() {
+    {
+        std::lock_guard<std::mutex> lock(stream_mutex());
+        if (stream_pool().size() < kPooledStreams) {
+            stream_pool().push_back({device, stream});
+            return;
+        }
+    }
+    cudaStreamDestroy(stream);
+}
+
 std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc* bvh,
                                     const mr_build_settings* build) {
     int device_count = 0;
@@ -632,11 +677,7 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
     }
 
     // Construction runs on its own stream with stream-ordered buffers (see AllocationScope).
-    struct OwnedStream {
-        cudaStream_t stream = nullptr;
-        OwnedStream() { MR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
-        ~OwnedStream() { cudaStreamDestroy(stream); }
-    } owned;
+    CallStream      owned;
     cudaStream_t    stream = owned.stream;
     AllocationScope scope(stream);
     size_t          bytes = 0;

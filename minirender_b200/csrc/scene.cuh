@@ -14,6 +14,19 @@ namespace mr {
 // keeps up to 2 GB of freed memory for reuse).
 cudaMemPool_t library_pool();
 
+// A non-blocking stream of the current device for the length of a call. Streams are pooled per
+// process (creating and destroying one takes 150-300 us, most of a small call): a call returns its
+// stream with its work done or ordered on it, and at most kPooledStreams wait for the next calls.
+constexpr size_t kPooledStreams = 32;
+struct CallStream {
+    cudaStream_t stream = nullptr;
+    int          device = 0;
+    CallStream();
+    ~CallStream();
+    CallStream(const CallStream&)            = delete;
+    CallStream& operator=(const CallStream&) = delete;
+};
+
 // While an AllocationScope is alive on a thread, DeviceBuffers allocated on that thread come from
 // the library pool, ordered on the scope's stream, and those released inside the same scope are
 // freed ordered on it too: no device-wide synchronisation, so scene construction can run beside

@@ -49,8 +49,7 @@ constexpr size_t kScratchBytes =
     2 * align256(kStaticPaths * sizeof(uint32_t)) +
     align256(kStaticPaths * kBinCount * sizeof(uint32_t)) + align256(kStaticPaths * sizeof(uint32_t)) +
     align256((kStaticBounces + 2) * sizeof(BounceCounters)) +
-    align256(kStatCount * sizeof(unsigned long long)) + align256(sizeof(unsigned)) +
-    align256(2 * kStaticPaths * sizeof(float4)) + align256(sizeof(unsigned));
+    align256(kStatisticsBytes) + align256(2 * kStaticPaths * sizeof(float4)) + align256(sizeof(unsigned));
 
 static __device__ __align__(256) unsigned char g_trace_scratch[kScratchBytes];
 
@@ -90,8 +89,7 @@ void carve(unsigned char* base, Workspace& ws, float4*& staging, unsigned*& inva
     ws.queues.bins       = reinterpret_cast<uint32_t*>(take(kStaticPaths * kBinCount * sizeof(uint32_t)));
     ws.queues.shadow     = reinterpret_cast<uint32_t*>(take(kStaticPaths * sizeof(uint32_t)));
     ws.queues.counters   = reinterpret_cast<BounceCounters*>(take((kStaticBounces + 2) * sizeof(BounceCounters)));
-    ws.queues.stats      = reinterpret_cast<unsigned long long*>(take(kStatCount * sizeof(unsigned long long)));
-    ws.queues.error      = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
+    ws.queues.set_statistics(take(kStatisticsBytes));
     staging              = reinterpret_cast<float4*>(take(2 * kStaticPaths * sizeof(float4)));
     invalid              = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
     if (offset > kScratchBytes) {

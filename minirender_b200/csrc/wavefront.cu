@@ -1173,6 +1173,19 @@ Workspace::~Workspace() {
 
 namespace {
 
+std::mutex                              pool_mutex;
+std::vector<std::shared_ptr<Workspace>> pool;  // least recently used first
+
+constexpr size_t kPooledWorkspaces     = 16;
+constexpr size_t kPooledWorkspaceBytes = size_t(12) << 30;  // four lanes of 8M paths and some small ones
+
+void drop_pooled_workspaces() {
+    std::vector<std::shared_ptr<Workspace>> dropped;
+    std::lock_guard<std::mutex>             lock(pool_mutex);
+    dropped.swap(pool);
+}
+
+
 std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     auto   ws     = std::make_shared<Workspace>();
     size_t offset = 0;
@@ -1193,11 +1206,14 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
     const size_t o_skeys  = field(capacity * sizeof(uint32_t));
     const size_t o_buck  = field((4 * kSortBuckets + 2 * kSortScanBlocks) * sizeof(uint32_t));
     const size_t o_ctr = field((max_bounces + 2) * sizeof(BounceCounters));
-    const size_t o_stats = field(kStatCount * sizeof(unsigned long long));
-    const size_t o_err = field(sizeof(unsigned));
+    const size_t o_stats = field(kStatisticsBytes);
     const size_t o_acc = field(2 * pixels * sizeof(float4));
     void*        mem   = nullptr;
-    MR_CUDA(cudaMalloc(&mem, offset));
+    if (cudaMalloc(&mem, offset) == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();  // not a sticky error: pooled workspaces may make room
+        drop_pooled_workspaces();
+        MR_CUDA(cudaMalloc(&mem, offset));
+    }
     char* base              = static_cast<char*>(mem);
     ws->memory              = mem;
     ws->bytes               = offset;
@@ -1217,22 +1233,19 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
     ws->queues.buckets      = reinterpret_cast<uint32_t*>(base + o_buck);
     MR_CUDA(cudaMemset(ws->queues.buckets, 0, 2 * kSortBuckets * sizeof(uint32_t)));
     ws->queues.counters     = reinterpret_cast<BounceCounters*>(base + o_ctr);
-    ws->queues.stats        = reinterpret_cast<unsigned long long*>(base + o_stats);
-    ws->queues.error        = reinterpret_cast<unsigned*>(base + o_err);
+    ws->queues.set_statistics(base + o_stats);
     ws->accumulator         = reinterpret_cast<float4*>(base + o_acc);
     return ws;
 }
-
-std::mutex                              pool_mutex;
-std::vector<std::shared_ptr<Workspace>> pool;
 
 }  // namespace
 
 // Workspaces are pooled per process: a request takes the smallest pooled workspace of its device
 // that is large enough in every dimension, and requests are rounded up (powers of two, bounces to
-// a multiple of 16) so that one workspace serves many job shapes. When more than four are pooled
-// the smallest goes: large ones serve every smaller request, so a stream of uneven jobs settles
-// on reuse instead of reallocating (a device-wide synchronising cudaFree each time).
+// a multiple of 16) so that one workspace serves many job shapes. Above kPooledWorkspaces or
+// kPooledWorkspaceBytes the least recently used go (when the smallest went, a shape that a few
+// larger ones did not cover was allocated and freed on every call: 3.6 ms of a 22 ms frame), and
+// all of them go when an allocation fails.
 std::shared_ptr<Workspace> acquire_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     int device = 0;
     MR_CUDA(cudaGetDevice(&device));
@@ -1271,27 +1284,29 @@ void release_workspace(std::shared_ptr<Workspace> ws) {
     if (!ws) {
         return;
     }
-    std::lock_guard<std::mutex> lock(pool_mutex);
+    std::vector<std::shared_ptr<Workspace>> dropped;  // freed (a device-wide wait) outside the lock
+    std::lock_guard<std::mutex>             lock(pool_mutex);
     pool.push_back(std::move(ws));
-    if (pool.size() > 4) {
-        auto smallest = std::min_element(pool.begin(), pool.end(), [](const auto& a, const auto& b) {
-            return a->bytes < b->bytes;
-        });
-        pool.erase(smallest);
+    size_t bytes = 0;
+    for (const auto& w : pool) {
+        bytes += w->bytes;
+    }
+    while (pool.size() > 1 && (pool.size() > kPooledWorkspaces || bytes > kPooledWorkspaceBytes)) {
+        bytes -= pool.front()->bytes;
+        dropped.push_back(std::move(pool.front()));
+        pool.erase(pool.begin());
     }
 }
 
 void reset_statistics(Workspace& ws, cudaStream_t stream) {
-    MR_CUDA(cudaMemsetAsync(ws.queues.stats, 0, kStatCount * sizeof(unsigned long long), stream));
-    MR_CUDA(cudaMemsetAsync(ws.queues.error, 0, sizeof(unsigned), stream));
+    MR_CUDA(cudaMemsetAsync(ws.queues.stats, 0, kStatisticsBytes, stream));
 }
 
 void read_statistics(Workspace& ws, cudaStream_t stream, mr_path_statistics* out, unsigned* error) {
-    unsigned long long stats[kStatCount];
-    unsigned           e = 0;
-    MR_CUDA(cudaMemcpyAsync(stats, ws.queues.stats, sizeof(stats), cudaMemcpyDeviceToHost, stream));
-    MR_CUDA(cudaMemcpyAsync(&e, ws.queues.error, sizeof(e), cudaMemcpyDeviceToHost, stream));
+    unsigned long long stats[kStatisticsBytes / sizeof(unsigned long long)];
+    MR_CUDA(cudaMemcpyAsync(stats, ws.queues.stats, kStatisticsBytes, cudaMemcpyDeviceToHost, stream));
     MR_CUDA(cudaStreamSynchronize(stream));
+    const unsigned e = static_cast<unsigned>(stats[kStatCount]);
     if (out) {
         std::memset(out, 0, sizeof(*out));
         out->paths                    = stats[kStatPaths];
@@ -1643,15 +1658,13 @@ void render_frame(const Scene& scene, const IntegratorParams& params, const mr_r
     // The extra workspaces go back to the pool only once the frame has finished; after an error
     // they are freed (cudaFree waits for the work still queued on them).
     struct MoreLanes {
-        std::shared_ptr<Workspace> ws[kFrameLanes - 1];
-        TileLane                   lanes[kFrameLanes - 1];
-        uint32_t                   count    = 0;
-        bool                       finished = false;
+        std::shared_ptr<Workspace>  ws[kFrameLanes - 1];
+        std::unique_ptr<CallStream> streams[kFrameLanes - 1];
+        TileLane                    lanes[kFrameLanes - 1];
+        uint32_t                    count    = 0;
+        bool                        finished = false;
         ~MoreLanes() {
             for (uint32_t i = 0; i < count; ++i) {
-                if (lanes[i].stream) {
-                    cudaStreamDestroy(lanes[i].stream);
-                }
                 if (finished) {
                     release_workspace(ws[i]);
                 }
@@ -1674,7 +1687,8 @@ void render_frame(const Scene& scene, const IntegratorParams& params, const mr_r
             }
             more.lanes[i].ws = more.ws[i].get();
             ++more.count;
-            MR_CUDA(cudaStreamCreateWithFlags(&more.lanes[i].stream, cudaStreamNonBlocking));
+            more.streams[i]      = std::make_unique<CallStream>();
+            more.lanes[i].stream = more.streams[i]->stream;
             reset_statistics(*more.ws[i], stream);
         }
     }

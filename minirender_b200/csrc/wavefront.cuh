@@ -42,6 +42,8 @@ enum Stat : int {
     kStatCount
 };
 
+constexpr size_t kStatisticsBytes = (kStatCount + 1) * sizeof(unsigned long long);  // and the error word
+
 struct IntegratorParams {
     uint32_t mode;
     uint32_t maximum_depth;
@@ -193,7 +195,11 @@ struct Queues {
     uint32_t*       shadow;
     BounceCounters* counters;  // maximum_depth + 2 entries
     unsigned long long* stats;  // kStatCount
-    unsigned*           error;
+    unsigned*           error;  // follows the statistics: one copy reads both
+    void set_statistics(void* block) {  // kStatisticsBytes of device memory
+        stats = static_cast<unsigned long long*>(block);
+        error = reinterpret_cast<unsigned*>(stats + kStatCount);
+    }
 };
 
 // Device workspace for `capacity` concurrent paths; pooled and reused across renders.

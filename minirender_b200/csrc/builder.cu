@@ -11,13 +11,14 @@
 //  - nodes with more than kSmallTask primitives are processed one level at a time by the whole
 //    GPU: fixed-size chunks of a node's primitive range reduce bounds and bin in shared memory
 //    and merge with one atomic per value per chunk; splits are chosen one warp per node;
-//    primitives are scattered with a chunk scan so the order is deterministic;
+//    primitives are scattered with a chunk scan so the order is deterministic. One block lists a
+//    level's chunks and emits the next level's tasks in order, so the host reads three numbers per
+//    level and sorts nothing;
 //  - smaller nodes are finished by one warp each, depth-first in shared memory, with node
 //    indices taken from a range reserved per subtree (unused indices are squeezed out at the end).
 // All arithmetic is FP32. Surface areas are evaluated on extents scaled by a power of two so the
 // products cannot overflow (the reference uses double for the same reason, intersection.cpp:44-50).
 #include <algorithm>
-#include <vector>
 
 #include "errors.hpp"
 #include "scan.cuh"
@@ -116,8 +117,11 @@ __global__ void init_task_state(TaskBounds* bounds, TaskBins* bins, uint32_t cou
 }
 
 // Pass 1: node bounds and centroid bounds.
-__global__ void reduce_bounds_kernel(const Chunk* chunks, const uint32_t* order, const float4* plo,
+__global__ void reduce_bounds_kernel(const Chunk* chunks, const uint32_t* chunk_total, const uint32_t* order, const float4* plo,
                                      const float4* phi, const float4* pc, TaskBounds* bounds) {
+    if (blockIdx.x >= *chunk_total) {
+        return;
+    }
     __shared__ uint32_t s[12];
     const Chunk ch = chunks[blockIdx.x];
     if (threadIdx.x < 12) {
@@ -161,9 +165,12 @@ __global__ void reduce_bounds_kernel(const Chunk* chunks, const uint32_t* order,
 }
 
 // Pass 2: 12 bins per axis.
-__global__ void bin_kernel(const Chunk* chunks, const uint32_t* order, const float4* plo,
+__global__ void bin_kernel(const Chunk* chunks, const uint32_t* chunk_total, const uint32_t* order, const float4* plo,
                            const float4* phi, const float4* pc, const TaskBounds* bounds,
                            TaskBins* bins) {
+    if (blockIdx.x >= *chunk_total) {
+        return;
+    }
     __shared__ uint32_t count[3][kBins];
     __shared__ uint32_t box[3][kBins][6];
     const Chunk ch = chunks[blockIdx.x];
@@ -292,8 +299,8 @@ __device__ __forceinline__ void write_node(mr_bvh_node& n, const float* lo, cons
 
 // Pass 3: one warp per large task decides leaf or split and writes leaves.
 __global__ void split_kernel(const Task* tasks, uint32_t count, const TaskBounds* bounds,
-                             const TaskBins* bins, Split* splits, uint32_t* child_counts,
-                             mr_bvh_node* nodes, unsigned long long* leaves, unsigned* depth) {
+                             const TaskBins* bins, Split* splits, mr_bvh_node* nodes,
+                             unsigned long long* leaves, unsigned* depth) {
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= count) {
         return;
@@ -315,8 +322,7 @@ __global__ void split_kernel(const Task* tasks, uint32_t count, const TaskBounds
         return;
     }
     atomicMax(depth, task.depth);
-    splits[t]       = s;
-    child_counts[t] = s.axis < 0 ? 0u : 2u;
+    splits[t] = s;
     if (s.axis < 0) {
         write_node(nodes[task.node], lo, hi, task.begin, 0, n);
         atomicAdd(leaves, 1ull);
@@ -326,8 +332,11 @@ __global__ void split_kernel(const Task* tasks, uint32_t count, const TaskBounds
 }
 
 // Pass 4: per chunk, how many primitives go left.
-__global__ void count_left_kernel(const Chunk* chunks, const uint32_t* order, const float4* pc,
+__global__ void count_left_kernel(const Chunk* chunks, const uint32_t* chunk_total, const uint32_t* order, const float4* pc,
                                   const TaskBounds* bounds, const Split* splits, uint32_t* left) {
+    if (blockIdx.x >= *chunk_total) {
+        return;
+    }
     __shared__ uint32_t total;
     const Chunk ch = chunks[blockIdx.x];
     const Split s  = splits[ch.task];
@@ -358,10 +367,13 @@ __global__ void count_left_kernel(const Chunk* chunks, const uint32_t* order, co
 }
 
 // Pass 5: stable scatter into `out` (chunks of split tasks only; others copy through).
-__global__ void scatter_kernel(const Chunk* chunks, const uint32_t* chunk_left_offset,
+__global__ void scatter_kernel(const Chunk* chunks, const uint32_t* chunk_total, const uint32_t* chunk_left_offset,
                                const uint32_t* task_first_chunk, const Task* tasks,
                                const uint32_t* order, const float4* pc, const TaskBounds* bounds,
                                const Split* splits, uint32_t* out) {
+    if (blockIdx.x >= *chunk_total) {
+        return;
+    }
     const Chunk    ch   = chunks[blockIdx.x];
     const Split    s    = splits[ch.task];
     const Task     task = tasks[ch.task];
@@ -401,75 +413,135 @@ __global__ void scatter_kernel(const Chunk* chunks, const uint32_t* chunk_left_o
     }
 }
 
-__global__ void copy_kernel(const Chunk* chunks, const uint32_t* in, uint32_t* out) {
+__global__ void copy_kernel(const Chunk* chunks, const uint32_t* chunk_total, const uint32_t* in, uint32_t* out) {
+    if (blockIdx.x >= *chunk_total) {
+        return;
+    }
     const Chunk ch = chunks[blockIdx.x];
     for (uint32_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
         out[i] = in[i];
     }
 }
 
-// Pass 6: link children, enqueue them as large or small tasks.
-__global__ void emit_children_kernel(const Task* tasks, uint32_t count, const Split* splits,
-                                     const uint32_t* child_offsets, uint32_t node_base,
-                                     mr_bvh_node* nodes, Task* next_large, uint32_t* next_large_count,
-                                     Task* small, uint32_t* small_count) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count || splits[t].axis < 0) {
-        return;
-    }
-    const Task&    task  = tasks[t];
-    const uint32_t left  = node_base + child_offsets[t];
-    const uint32_t right = left + 1;
-    nodes[task.node].first = left;
-    nodes[task.node].right = right;
-    const uint32_t mid     = task.begin + splits[t].left_count;
-    const Task     children[2] = {{task.begin, mid, left, task.depth + 1, 0},
-                                  {mid, task.end, right, task.depth + 1, 0}};
-    for (int c = 0; c < 2; ++c) {
-        const uint32_t n = children[c].end - children[c].begin;
-        if (n > kSmallTask) {  // at depth 48 the split pass turns it into a leaf
-            next_large[atomicAdd(next_large_count, 1u)] = children[c];
-        } else {
-            small[atomicAdd(small_count, 1u)] = children[c];
+// What the host reads after a level.
+struct LevelState {
+    uint32_t large;  // tasks of the next level
+    uint32_t small;  // small tasks so far
+    uint32_t nodes;  // nodes so far
+};
+
+// Pass 6, one block: links the children of every split task and lists them as tasks of the next level
+// or small tasks, left before right in task order (so tasks stay sorted by where they begin).
+__global__ void __launch_bounds__(1024)
+emit_children_kernel(const Task* tasks, uint32_t count, const Split* splits, mr_bvh_node* nodes,
+                     Task* next_large, Task* small, LevelState* state) {
+    uint32_t large_base = 0, small_base = state->small, node_base = state->nodes;
+    for (uint32_t base = 0; base < count; base += blockDim.x) {
+        const uint32_t t = base + threadIdx.x;
+        Task           children[2];
+        bool           split = t < count && splits[t].axis >= 0;
+        uint32_t       large = 0;
+        if (split) {
+            const Task     task = tasks[t];
+            const uint32_t mid  = task.begin + splits[t].left_count;
+            children[0]         = {task.begin, mid, 0, task.depth + 1, 0};
+            children[1]         = {mid, task.end, 0, task.depth + 1, 0};
+            for (int c = 0; c < 2; ++c) {  // at depth 48 the split pass turns a large one into a leaf
+                large += children[c].end - children[c].begin > kSmallTask ? 1u : 0u;
+            }
         }
+        uint32_t       total;  // children in the low half, large ones in the high half
+        const uint32_t rank = block_exclusive_scan(split ? 2u | large << 16 : 0u, total);
+        if (split) {
+            const uint32_t first = node_base + (rank & 0xffffu);
+            uint32_t       l = large_base + (rank >> 16), m = small_base + (rank & 0xffffu) - (rank >> 16);
+            nodes[tasks[t].node].first = first;
+            nodes[tasks[t].node].right = first + 1;
+            for (uint32_t c = 0; c < 2; ++c) {
+                children[c].node = first + c;
+                if (children[c].end - children[c].begin > kSmallTask) {
+                    next_large[l++] = children[c];
+                } else {
+                    small[m++] = children[c];
+                }
+            }
+        }
+        node_base += total & 0xffffu;
+        large_base += total >> 16;
+        small_base += (total & 0xffffu) - (total >> 16);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *state = {large_base, small_base, node_base};
     }
 }
 
-// Chunk descriptors for a level.
-__global__ void make_chunks_kernel(const Task* tasks, uint32_t count, const uint32_t* chunk_offsets,
-                                   Chunk* chunks, uint32_t* task_first_chunk) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) {
-        return;
+// One block: the chunks of a level's tasks, and how many there are.
+__global__ void __launch_bounds__(1024)
+make_chunks_kernel(const Task* tasks, uint32_t count, Chunk* chunks, uint32_t* task_first_chunk,
+                   uint32_t* chunk_total) {
+    uint32_t running = 0;
+    for (uint32_t base = 0; base < count; base += blockDim.x) {
+        const uint32_t t = base + threadIdx.x;
+        Task           task{};
+        if (t < count) {
+            task = tasks[t];
+        }
+        uint32_t total;
+        uint32_t k = running + block_exclusive_scan((task.end - task.begin + kChunk - 1) / kChunk, total);
+        if (t < count) {
+            task_first_chunk[t] = k;
+            for (uint32_t b = task.begin; b < task.end; b += kChunk, ++k) {
+                chunks[k] = {t, b, min(b + kChunk, task.end)};
+            }
+        }
+        running += total;
     }
-    const Task&    task  = tasks[t];
-    const uint32_t first = chunk_offsets[t];
-    task_first_chunk[t]  = first;
-    uint32_t k           = first;
-    for (uint32_t b = task.begin; b < task.end; b += kChunk, ++k) {
-        chunks[k] = {t, b, min(b + kChunk, task.end)};
+    if (threadIdx.x == 0) {
+        *chunk_total = running;
     }
 }
 
-__global__ void chunk_count_kernel(const Task* tasks, uint32_t count, uint32_t* out) {
+// One block: exclusive scan of the chunks' left counts.
+__global__ void __launch_bounds__(1024)
+scan_left_kernel(const uint32_t* left, const uint32_t* chunk_total, uint32_t* offsets) {
+    const uint32_t n       = *chunk_total;
+    uint32_t       running = 0;
+    for (uint32_t base = 0; base < n; base += blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        uint32_t       total;
+        const uint32_t rank = block_exclusive_scan(i < n ? left[i] : 0u, total);
+        if (i < n) {
+            offsets[i] = running + rank;
+        }
+        running += total;
+    }
+}
+
+// Small tasks in the order of where they begin: a mark per first primitive, scanned, is their rank.
+__global__ void mark_small_kernel(const Task* small, uint32_t count, uint32_t* marks) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < count) {
-        out[t] = (tasks[t].end - tasks[t].begin + kChunk - 1) / kChunk;
+        marks[small[t].begin] = 1;
     }
 }
 
-__global__ void small_reserve_kernel(const Task* small, uint32_t count, uint32_t* sizes) {
+// Moves each small task to its rank, with the node indices its descendants may take (pre-order).
+__global__ void sort_small_kernel(const Task* small, uint32_t count, const uint32_t* ranks, Task* sorted,
+                                  uint32_t* sizes) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < count) {
-        const uint32_t n = small[t].end - small[t].begin;
-        sizes[t]         = 2 * n - 2;  // descendants of a subtree over n primitives
+        const Task     task = small[t];
+        const uint32_t r    = ranks[task.begin];
+        sorted[r]           = task;
+        sizes[r]            = 2 * (task.end - task.begin) - 2;  // descendants of a subtree over n primitives
     }
 }
 
 // Small subtrees: one warp per task, depth-first in shared memory. Node indices are assigned in
 // pre-order from the task's reserved range (the reference's emplacement order, bvh.cpp:104-105).
 __global__ void __launch_bounds__(32 * kSmallWarps)
-small_build_kernel(const Task* small, uint32_t count, const uint32_t* ranges, uint32_t range_base,
+small_build_kernel(const Task* small, uint32_t count, const uint32_t* ranges, const LevelState* state,
                    uint32_t* order, const float4* plo, const float4* phi, const float4* pc,
                    mr_bvh_node* nodes, unsigned long long* leaves, unsigned* max_depth) {
     struct Entry {
@@ -491,7 +563,7 @@ small_build_kernel(const Task* small, uint32_t count, const uint32_t* ranges, ui
         s_idx[warp][i] = order[task.begin + i];
     }
     __syncwarp();
-    uint32_t next_node = range_base + ranges[t];
+    uint32_t next_node = state->nodes + ranges[t];
     int      sp        = 0;
     if (lane == 0) {
         s_stack[warp][0] = {0, n, task.depth, kUnusedNode};
@@ -632,13 +704,6 @@ small_build_kernel(const Task* small, uint32_t count, const uint32_t* ranges, ui
         atomicAdd(leaves, static_cast<unsigned long long>(local_leaves));
         atomicMax(max_depth, local_depth);
     }
-    // Mark the unused tail of the reserved range.
-    const uint32_t reserved_end = range_base + ranges[t] + (2 * n - 2);
-    for (uint32_t k = next_node + lane; k < reserved_end; k += 32) {
-        nodes[k].count = kUnusedNode;
-        nodes[k].first = 0;
-        nodes[k].right = 0;
-    }
 }
 
 __global__ void valid_flag_kernel(const mr_bvh_node* nodes, uint32_t count, uint32_t* flags) {
@@ -701,9 +766,9 @@ BuildResult build_bvh_device(const float4* lo, const float4* hi, const float4* c
     DeviceBuffer<uint8_t> raw;
     const size_t bytes =
         2 * max_tasks * sizeof(Task) + max_tasks * (sizeof(TaskBounds) + sizeof(TaskBins) + sizeof(Split)) +
-        6 * max_tasks * sizeof(uint32_t) + max_chunks * (sizeof(Chunk) + 2 * sizeof(uint32_t)) +
+        max_tasks * sizeof(uint32_t) + max_chunks * (sizeof(Chunk) + 2 * sizeof(uint32_t)) +
         static_cast<size_t>(count) * (sizeof(Task) + 2 * sizeof(uint32_t)) + 64 * 16 +
-        (scan_scratch_size(std::max(max_chunks, static_cast<size_t>(count))) + 8) * sizeof(uint32_t);
+        (scan_scratch_size(node_capacity) + 8) * sizeof(uint32_t);
     raw.allocate(bytes);
     uint8_t* cursor = raw.ptr;
     const auto take = [&](size_t b) {
@@ -716,10 +781,6 @@ BuildResult build_bvh_device(const float4* lo, const float4* hi, const float4* c
     TaskBounds* task_bounds   = reinterpret_cast<TaskBounds*>(take(max_tasks * sizeof(TaskBounds)));
     TaskBins*   task_bins     = reinterpret_cast<TaskBins*>(take(max_tasks * sizeof(TaskBins)));
     Split*      splits        = reinterpret_cast<Split*>(take(max_tasks * sizeof(Split)));
-    uint32_t*   child_counts  = reinterpret_cast<uint32_t*>(take(max_tasks * sizeof(uint32_t)));
-    uint32_t*   child_offsets = reinterpret_cast<uint32_t*>(take(max_tasks * sizeof(uint32_t)));
-    uint32_t*   chunk_counts  = reinterpret_cast<uint32_t*>(take(max_tasks * sizeof(uint32_t)));
-    uint32_t*   chunk_offsets = reinterpret_cast<uint32_t*>(take(max_tasks * sizeof(uint32_t)));
     uint32_t*   task_first    = reinterpret_cast<uint32_t*>(take(max_tasks * sizeof(uint32_t)));
     Chunk*      chunks        = reinterpret_cast<Chunk*>(take(max_chunks * sizeof(Chunk)));
     uint32_t*   chunk_left    = reinterpret_cast<uint32_t*>(take(max_chunks * sizeof(uint32_t)));
@@ -730,111 +791,92 @@ BuildResult build_bvh_device(const float4* lo, const float4* hi, const float4* c
     uint32_t*   counters      = reinterpret_cast<uint32_t*>(take(16 * sizeof(uint32_t)));
     unsigned long long* leaves = reinterpret_cast<unsigned long long*>(take(sizeof(unsigned long long)));
     uint32_t*   scratch       = reinterpret_cast<uint32_t*>(
-        take((scan_scratch_size(std::max(max_chunks, static_cast<size_t>(count))) + 8) * sizeof(uint32_t)));
-    // counters: [0] next large count, [1] small count, [2] child total, [3] chunk total,
-    //           [4] max depth, [5] small range total
+        take((scan_scratch_size(node_capacity) + 8) * sizeof(uint32_t)));
+    // counters: [0-2] LevelState, [3] chunks of the level, [4] maximum depth, [6] nodes in use
+    LevelState* state       = reinterpret_cast<LevelState*>(counters);
+    uint32_t*   chunk_total = counters + 3;
     MR_CUDA(cudaMemsetAsync(counters, 0, 16 * sizeof(uint32_t), stream));
     MR_CUDA(cudaMemsetAsync(leaves, 0, sizeof(unsigned long long), stream));
+    // Every node index is unused (count kUnusedNode) until a node takes it.
+    MR_CUDA(cudaMemsetAsync(nodes.ptr, 0xff, node_capacity * sizeof(mr_bvh_node), stream));
 
-    uint32_t node_base = 1;  // node 0 is the root
     uint32_t level_count = 0;
     uint32_t small_total = 0;
-    // Root task: large unless it is small enough for one warp.
-    const Task root{0, count, 0, 0, 0};
-    int        cur = 0;
+    // Root task (node 0): large unless it is small enough for one warp.
+    const Task       root{0, count, 0, 0, 0};
+    const LevelState first{0, count > kSmallTask ? 0u : 1u, 1};
+    int              cur = 0;
+    MR_CUDA(cudaMemcpyAsync(state, &first, sizeof(first), cudaMemcpyHostToDevice, stream));
     if (count > kSmallTask) {
         MR_CUDA(cudaMemcpyAsync(tasks[0], &root, sizeof(Task), cudaMemcpyHostToDevice, stream));
         level_count = 1;
     } else {
         MR_CUDA(cudaMemcpyAsync(small, &root, sizeof(Task), cudaMemcpyHostToDevice, stream));
         small_total = 1;
-        const uint32_t one = 1;
-        MR_CUDA(cudaMemcpyAsync(counters + 1, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
     }
 
     while (level_count > 0) {
         Task* level = tasks[cur];
         Task* next  = tasks[cur ^ 1];
-        // Chunk list of this level.
-        chunk_count_kernel<<<blocks_for(level_count), 256, 0, stream>>>(level, level_count, chunk_counts);
-        exclusive_scan(chunk_counts, chunk_offsets, level_count, scratch, counters + 3, stream);
-        make_chunks_kernel<<<blocks_for(level_count), 256, 0, stream>>>(level, level_count, chunk_offsets,
-                                                                          chunks, task_first);
-        uint32_t chunk_total = 0;
-        MR_CUDA(cudaMemcpyAsync(&chunk_total, counters + 3, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        MR_CUDA(cudaStreamSynchronize(stream));
+        // At most this many chunks; the blocks beyond the level's own count leave at once.
+        const unsigned grid = static_cast<unsigned>(std::min<size_t>(max_chunks, count / kChunk + level_count));
+        make_chunks_kernel<<<1, 1024, 0, stream>>>(level, level_count, chunks, task_first, chunk_total);
         init_task_state<<<level_count, 128, 0, stream>>>(task_bounds, task_bins, level_count);
-        reduce_bounds_kernel<<<chunk_total, 256, 0, stream>>>(chunks, order.ptr, lo, hi, centroid, task_bounds);
-        bin_kernel<<<chunk_total, 256, 0, stream>>>(chunks, order.ptr, lo, hi, centroid, task_bounds, task_bins);
+        reduce_bounds_kernel<<<grid, 256, 0, stream>>>(chunks, chunk_total, order.ptr, lo, hi, centroid, task_bounds);
+        bin_kernel<<<grid, 256, 0, stream>>>(chunks, chunk_total, order.ptr, lo, hi, centroid, task_bounds, task_bins);
         split_kernel<<<blocks_for(level_count, 4), 128, 0, stream>>>(level, level_count, task_bounds, task_bins,
-                                                                       splits, child_counts, nodes.ptr, leaves,
-                                                                       counters + 4);
-        count_left_kernel<<<chunk_total, 256, 0, stream>>>(chunks, order.ptr, centroid, task_bounds, splits,
-                                                            chunk_left);
-        exclusive_scan(chunk_left, chunk_left_off, chunk_total, scratch, nullptr, stream);
-        scatter_kernel<<<chunk_total, 256, 0, stream>>>(chunks, chunk_left_off, task_first, level, order.ptr,
-                                                         centroid, task_bounds, splits, scratch_order.ptr);
-        copy_kernel<<<chunk_total, 256, 0, stream>>>(chunks, scratch_order.ptr, order.ptr);
-        exclusive_scan(child_counts, child_offsets, level_count, scratch, counters + 2, stream);
-        MR_CUDA(cudaMemsetAsync(counters, 0, sizeof(uint32_t), stream));
-        emit_children_kernel<<<blocks_for(level_count), 256, 0, stream>>>(level, level_count, splits,
-                                                                           child_offsets, node_base, nodes.ptr,
-                                                                           next, counters, small, counters + 1);
+                                                                     splits, nodes.ptr, leaves, counters + 4);
+        count_left_kernel<<<grid, 256, 0, stream>>>(chunks, chunk_total, order.ptr, centroid, task_bounds, splits,
+                                                    chunk_left);
+        scan_left_kernel<<<1, 1024, 0, stream>>>(chunk_left, chunk_total, chunk_left_off);
+        scatter_kernel<<<grid, 256, 0, stream>>>(chunks, chunk_total, chunk_left_off, task_first, level, order.ptr,
+                                                 centroid, task_bounds, splits, scratch_order.ptr);
+        copy_kernel<<<grid, 256, 0, stream>>>(chunks, chunk_total, scratch_order.ptr, order.ptr);
+        emit_children_kernel<<<1, 1024, 0, stream>>>(level, level_count, splits, nodes.ptr, next, small, state);
         MR_CUDA(cudaGetLastError());
-        uint32_t host_counters[3];
-        MR_CUDA(cudaMemcpyAsync(host_counters, counters, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+        LevelState host{};
+        MR_CUDA(cudaMemcpyAsync(&host, state, sizeof(host), cudaMemcpyDeviceToHost, stream));
         MR_CUDA(cudaStreamSynchronize(stream));
-        node_base += host_counters[2];
-        level_count = host_counters[0];
-        small_total = host_counters[1];
-        // Deterministic task order for the next level and the small list: by range begin.
-        if (level_count > 1) {
-            std::vector<Task> h(level_count);
-            MR_CUDA(cudaMemcpyAsync(h.data(), next, level_count * sizeof(Task), cudaMemcpyDeviceToHost, stream));
-            MR_CUDA(cudaStreamSynchronize(stream));
-            std::sort(h.begin(), h.end(), [](const Task& a, const Task& b) { return a.begin < b.begin; });
-            MR_CUDA(cudaMemcpyAsync(next, h.data(), level_count * sizeof(Task), cudaMemcpyHostToDevice, stream));
-        }
+        level_count = host.large;
+        small_total = host.small;
         cur ^= 1;
     }
 
+    DeviceBuffer<Task> sorted;
     if (small_total > 0) {
-        std::vector<Task> h(small_total);
-        MR_CUDA(cudaMemcpyAsync(h.data(), small, small_total * sizeof(Task), cudaMemcpyDeviceToHost, stream));
-        MR_CUDA(cudaStreamSynchronize(stream));
-        std::sort(h.begin(), h.end(), [](const Task& a, const Task& b) { return a.begin < b.begin; });
-        MR_CUDA(cudaMemcpyAsync(small, h.data(), small_total * sizeof(Task), cudaMemcpyHostToDevice, stream));
-        small_reserve_kernel<<<blocks_for(small_total), 256, 0, stream>>>(small, small_total, small_sizes);
-        exclusive_scan(small_sizes, small_ranges, small_total, scratch, counters + 5, stream);
+        uint32_t* marks = scratch_order.ptr;
+        sorted.allocate(small_total);
+        MR_CUDA(cudaMemsetAsync(marks, 0, count * sizeof(uint32_t), stream));
+        mark_small_kernel<<<blocks_for(small_total), 256, 0, stream>>>(small, small_total, marks);
+        exclusive_scan(marks, marks, count, scratch, nullptr, stream);
+        sort_small_kernel<<<blocks_for(small_total), 256, 0, stream>>>(small, small_total, marks, sorted.ptr,
+                                                                        small_sizes);
+        exclusive_scan(small_sizes, small_ranges, small_total, scratch, nullptr, stream);
         const unsigned blocks = (small_total + kSmallWarps - 1) / kSmallWarps;
-        small_build_kernel<<<blocks, 32 * kSmallWarps, 0, stream>>>(small, small_total, small_ranges, node_base,
+        small_build_kernel<<<blocks, 32 * kSmallWarps, 0, stream>>>(sorted.ptr, small_total, small_ranges, state,
                                                                      order.ptr, lo, hi, centroid, nodes.ptr,
                                                                      leaves, counters + 4);
         MR_CUDA(cudaGetLastError());
-        uint32_t reserved = 0;
-        MR_CUDA(cudaMemcpyAsync(&reserved, counters + 5, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        MR_CUDA(cudaStreamSynchronize(stream));
-        node_base += reserved;
     }
 
     // Squeeze out unused node indices.
-    const uint32_t used_capacity = node_base;
+    const uint32_t used_capacity = static_cast<uint32_t>(node_capacity);
     DeviceBuffer<uint32_t> valid, index;
     valid.allocate(used_capacity);
     index.allocate(used_capacity);
     valid_flag_kernel<<<blocks_for(used_capacity), 256, 0, stream>>>(nodes.ptr, used_capacity, valid.ptr);
     exclusive_scan(valid.ptr, index.ptr, used_capacity, scratch, counters + 6, stream);
-    uint32_t compact = 0;
-    MR_CUDA(cudaMemcpyAsync(&compact, counters + 6, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    uint32_t           host_counters[16];
+    unsigned long long host_leaves = 0;
+    MR_CUDA(cudaMemcpyAsync(host_counters, counters, sizeof(host_counters), cudaMemcpyDeviceToHost, stream));
+    MR_CUDA(cudaMemcpyAsync(&host_leaves, leaves, sizeof(host_leaves), cudaMemcpyDeviceToHost, stream));
     MR_CUDA(cudaStreamSynchronize(stream));
+    const uint32_t compact    = host_counters[6];
+    const uint32_t host_depth = host_counters[4];
     result.nodes.allocate(compact);
     compact_nodes_kernel<<<blocks_for(used_capacity), 256, 0, stream>>>(nodes.ptr, used_capacity, index.ptr,
                                                                          result.nodes.ptr);
     MR_CUDA(cudaGetLastError());
-    unsigned long long host_leaves = 0;
-    uint32_t           host_depth  = 0;
-    MR_CUDA(cudaMemcpyAsync(&host_leaves, leaves, sizeof(host_leaves), cudaMemcpyDeviceToHost, stream));
-    MR_CUDA(cudaMemcpyAsync(&host_depth, counters + 4, sizeof(host_depth), cudaMemcpyDeviceToHost, stream));
     MR_CUDA(cudaEventRecord(stop, stream));
     MR_CUDA(cudaStreamSynchronize(stream));
     float ms = 0;

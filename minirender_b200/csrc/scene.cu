@@ -107,12 +107,21 @@ __device__ __forceinline__ float node_area(const mr_bvh_node& n) {
     return ex * ey + ey * ez + ez * ex;
 }
 
-__global__ void collapse_count_kernel(const mr_bvh_node* nodes, const uint32_t* roots, uint32_t count,
-                                      int4* children, uint32_t* interior_counts) {
+// A level of the collapse: how many wide nodes it has and the index of its first.
+struct CollapseLevel {
+    uint32_t count, base;
+};
+
+__global__ void collapse_count_kernel(const mr_bvh_node* nodes, const uint32_t* roots, const CollapseLevel* level,
+                                      uint32_t bound, int4* all_children, uint32_t* interior_counts) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) {
+    if (k >= level->count) {
+        if (k < bound) {
+            interior_counts[k] = 0;
+        }
         return;
     }
+    int4* children = all_children + level->base;
     const mr_bvh_node& root = nodes[roots[k]];
     int c[4] = {static_cast<int>(root.first), static_cast<int>(root.right), -1, -1};
     int n    = 2;
@@ -142,14 +151,17 @@ __global__ void collapse_count_kernel(const mr_bvh_node* nodes, const uint32_t* 
 }
 
 // Writes wide node `base + k` (layout in device_scene.cuh).
-__global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* children, uint32_t count,
-                                      const uint32_t* offsets, uint32_t base, uint32_t next_base,
-                                      float4* wide, uint32_t* next_roots) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* all_children, CollapseLevel* level,
+                                      const uint32_t* offsets, float4* wide, uint32_t* next_roots) {
+    const uint32_t k     = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t count = level->count, base = level->base, next_base = base + count;
+    if (k == 0) {
+        level[1].base = next_base;  // its count is the scan's total
+    }
     if (k >= count) {
         return;
     }
-    const int4 c4   = children[k];
+    const int4 c4   = all_children[base + k];
     const int  c[4] = {c4.x, c4.y, c4.z, c4.w};
     float      lo[3][4], hi[3][4];
     int        ref[4];
@@ -209,6 +221,13 @@ __global__ void mark_leaf_end_kernel(const mr_bvh_node* nodes, uint32_t count, f
     }
     float4& t = tris[3 * static_cast<size_t>(nodes[i].first + nodes[i].count - 1) + 1];
     t.w       = __uint_as_float(__float_as_uint(t.w) | kTriLeafEnd);
+}
+
+__global__ void scatter_emitters_kernel(const uint2* pairs, uint32_t count, uint32_t* prim_emitter) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) {
+        prim_emitter[pairs[i].x] = pairs[i].y;
+    }
 }
 
 bool finite3h(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1]) && std::isfinite(v[2]); }
@@ -381,22 +400,39 @@ WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t node_count, cudaSt
     offsets.allocate(interior);
     scratch.allocate(scan_scratch_size(interior));
     MR_CUDA(cudaMemsetAsync(roots[0].ptr, 0, sizeof(uint32_t), stream));  // the root
-    uint32_t level = 1, base = 0, cur = 0;
-    while (level > 0) {
-        int4* children = out.children.ptr + base;
-        collapse_count_kernel<<<(level + 127) / 128, 128, 0, stream>>>(ref_nodes, roots[cur].ptr, level,
-                                                                       children, counts.ptr);
-        exclusive_scan(counts.ptr, offsets.ptr, level, scratch.ptr, total.ptr, stream);
-        collapse_write_kernel<<<(level + 127) / 128, 128, 0, stream>>>(
-            ref_nodes, children, level, offsets.ptr, base, base + level, out.nodes.ptr, roots[cur ^ 1].ptr);
-        uint32_t next = 0;
-        MR_CUDA(cudaMemcpyAsync(&next, total.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        MR_CUDA(cudaStreamSynchronize(stream));
-        base += level;
-        level = next;
-        cur ^= 1;
+    // Levels run from counts on the device, a few at a time between the host's looks at them: at
+    // most 4^level nodes each, blocks beyond a level's own count leave at once. A wide level holds at
+    // least one binary level, so there are at most 64.
+    constexpr uint32_t          kMaxLevels = 64, kAhead = 4;
+    DeviceBuffer<CollapseLevel> levels;
+    levels.allocate(kMaxLevels + 2);
+    const CollapseLevel first{1, 0};
+    MR_CUDA(cudaMemsetAsync(levels.ptr, 0, (kMaxLevels + 2) * sizeof(CollapseLevel), stream));
+    MR_CUDA(cudaMemcpyAsync(levels.ptr, &first, sizeof(first), cudaMemcpyHostToDevice, stream));
+    uint32_t level = 0, bound = 1;
+    for (uint32_t look = 2; level < kMaxLevels; ++level) {
+        collapse_count_kernel<<<(bound + 127) / 128, 128, 0, stream>>>(ref_nodes, roots[level & 1].ptr,
+                                                                       levels.ptr + level, bound,
+                                                                       out.children.ptr, counts.ptr);
+        exclusive_scan(counts.ptr, offsets.ptr, bound, scratch.ptr, &levels.ptr[level + 1].count, stream);
+        collapse_write_kernel<<<(bound + 127) / 128, 128, 0, stream>>>(ref_nodes, out.children.ptr,
+                                                                       levels.ptr + level, offsets.ptr,
+                                                                       out.nodes.ptr, roots[(level + 1) & 1].ptr);
+        const bool full = bound == interior;
+        bound           = static_cast<uint32_t>(std::min<uint64_t>(4ull * bound, interior));
+        look            = full ? look - 1 : look;  // the first levels are full ones: no need to look
+        if (look == 0 || level + 1 == kMaxLevels) {
+            CollapseLevel next{};
+            MR_CUDA(cudaMemcpyAsync(&next, levels.ptr + level + 1, sizeof(next), cudaMemcpyDeviceToHost, stream));
+            MR_CUDA(cudaStreamSynchronize(stream));
+            out.count = next.base + next.count;
+            if (next.count == 0) {
+                break;
+            }
+            look = kAhead;
+        }
     }
-    out.count = base;
+    MR_CUDA(cudaGetLastError());
     return out;
 }
 
@@ -460,7 +496,7 @@ void build_light_table(Scene& scene, const mr_scene_desc& desc, const std::vecto
                        double map_integral, cudaStream_t stream) {
     LightTable&           t     = scene.light_table;
     const uint32_t        prims = scene.d.primitive_count;
-    std::vector<uint32_t> emitter_of_prim(std::max<uint32_t>(1, prims), kNone);
+    std::vector<uint2>    emitters;  // (primitive, light)
     t = LightTable{};
     for (uint32_t i = 0; i < desc.instance_count; ++i) {
         const mr_instance& in  = desc.instances[i];
@@ -491,7 +527,7 @@ void build_light_table(Scene& scene, const mr_scene_desc& desc, const std::vecto
             l.area         = area;
             l.kind         = kLightArea;
             l.double_sided = mat.double_sided;
-            emitter_of_prim[first_prim[i] + tri] = static_cast<uint32_t>(t.lights.size());
+            emitters.push_back(make_uint2(first_prim[i] + tri, static_cast<uint32_t>(t.lights.size())));
             t.lights.push_back(l);
             t.weights.push_back((mat.double_sided ? 2.0f : 1.0f) * kPi * area * luminance(radiance));
             t.scales.push_back(0);
@@ -523,10 +559,18 @@ void build_light_table(Scene& scene, const mr_scene_desc& desc, const std::vecto
         t.weights.push_back(integral);
         t.scales.push_back(1);
     }
-    scene.prim_emitter.allocate(emitter_of_prim.size());
-    MR_CUDA(cudaMemcpyAsync(scene.prim_emitter.ptr, emitter_of_prim.data(),
-                            emitter_of_prim.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-    MR_CUDA(cudaStreamSynchronize(stream));  // the source vector goes away with this function
+    // The map is all kNone but for the emitters: set on the device, then their entries scattered.
+    scene.prim_emitter.allocate(std::max<uint32_t>(1, prims));
+    MR_CUDA(cudaMemsetAsync(scene.prim_emitter.ptr, 0xff, std::max<uint32_t>(1, prims) * sizeof(uint32_t), stream));
+    if (!emitters.empty()) {
+        DeviceBuffer<uint2> pairs;
+        const uint32_t      n = static_cast<uint32_t>(emitters.size());
+        pairs.allocate(n);
+        MR_CUDA(cudaMemcpyAsync(pairs.ptr, emitters.data(), n * sizeof(uint2), cudaMemcpyHostToDevice, stream));
+        scatter_emitters_kernel<<<(n + 255) / 256, 256, 0, stream>>>(pairs.ptr, n, scene.prim_emitter.ptr);
+        MR_CUDA(cudaGetLastError());
+        MR_CUDA(cudaStreamSynchronize(stream));  // the source vector goes away with this function
+    }
     scene.d.prim_emitter = scene.prim_emitter.ptr;
 }
 

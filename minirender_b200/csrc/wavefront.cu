@@ -414,9 +414,9 @@ template <bool SHADOW, bool MEDIA, bool BATCH> struct QueueIo {
 // before this bounce's shading adds emission, the reference's accumulation order). Flattened
 // scenes are streamed (stream.cuh) with 8 resident blocks per SM (<= 64 registers; 7 blocks of 72
 // were 1-3% slower): the traversal waits on loads and more warps hide them. In a multi-job wave
-// (BATCH) every path finds its scene through its segment. With two-level scenes in the launch (TWO)
-// warps fetch 32 items at a time and the kernel carries the two-level traversal; it runs 5 blocks
-// per SM (<= 102 registers) so that its larger state stays in registers.
+// (BATCH) every path finds its scene through its segment. With two-level scenes in the launch, or few
+// rays per lane (TWO), warps fetch 32 items at a time and the kernel carries the two-level traversal;
+// it runs 5 blocks per SM (<= 102 registers) so that its larger state stays in registers.
 template <bool MEDIA, bool BATCH, bool TWO>
 __global__ void __launch_bounds__(kStreamBlock, TWO ? 5 : 8) trace_kernel(KernelArgs a) {
     BounceCounters* ctr      = a.q.counters + a.bounce;
@@ -1401,7 +1401,11 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
     KernelTiming&      timing = kernel_timing();
     bool               timed  = false;
     timed = timing.enabled.load();
-    note_launches(1 + (media && !two ? 3ull : 2ull) * (params.maximum_depth + 1) + (ray_sort ? 4ull * params.maximum_depth : 0ull) +
+    // Waves of few rays per lane do not stream (see kStreamMinPaths): the two-level scenes' kernel
+    // traces them too.
+    const bool streamed = !two && streams(init.count, scene.d.slot_count);
+    const int  traced   = (media ? 1 : 0) + (streamed ? 0 : 2);
+    note_launches(1 + (media && streamed ? 3ull : 2ull) * (params.maximum_depth + 1) + (ray_sort ? 4ull * params.maximum_depth : 0ull) +
                   (init.capture ? 1 : 0));
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
     // The timed launches are the trace kernels: nearest-hit and shadow tests both count.
@@ -1421,7 +1425,7 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
         }
         // The first shadow rays (queued by bounce 0's shading) are traced with bounce 1.
         a.occluded_out = bounce == 1 && init.capture ? init.capture->occluded : nullptr;
-        switch (variant) {
+        switch (traced) {
         case 0: trace_kernel<false, false, false><<<shape.trace_blocks[0], kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 1: trace_kernel<true, false, false><<<shape.trace_blocks[1], kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 2: trace_kernel<false, false, true><<<shape.trace_blocks[2], 128, 0, stream>>>(a); break;
@@ -1432,7 +1436,7 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
             cudaEventRecord(e1, stream);
             events.emplace_back(e0, e1);
         }
-        if (media && !two) {
+        if (media && streamed) {
             medium_kernel<false><<<shape.shade_blocks, 128, 0, stream>>>(a);
         }
         if (two) {
@@ -1483,7 +1487,7 @@ void Engine::batch_occupancy(int& trace_blocks_per_sm, int& shade_blocks_per_sm)
 }
 
 void Engine::enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, bool media, bool two,
-                                 bool ray_sort, const BatchShape& shape, Workspace& ws,
+                                 bool streamed, bool ray_sort, const BatchShape& shape, Workspace& ws,
                                  cudaStream_t stream) {
     if (maximum_depth + 1 > ws.max_bounces || !ws.state.segment) {
         fail(MR_LENGTH_ERROR, "Wave exceeds the workspace capacity");
@@ -1501,10 +1505,10 @@ void Engine::enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, b
     if (!ray_sort) {
         a.q.staging = nullptr;
     }
-    // The two-level variants keep fewer blocks resident (more registers per thread): their grid
-    // is capped at what fits, the persistent loop takes the work either way.
+    // The variants that do not stream keep fewer blocks resident (more registers per thread): their
+    // grid is capped at what fits, the persistent loop takes the work either way.
     int trace_blocks = shape.trace_blocks;
-    if (two) {
+    if (!streamed) {
         int per = 0;
         MR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &per, media ? trace_kernel<true, true, true> : trace_kernel<false, true, true>, 128, 0));
@@ -1514,13 +1518,13 @@ void Engine::enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, b
     init_batch_kernel<<<sms * 8, 256, 0, stream>>>(a);
     for (uint32_t bounce = 0; bounce <= maximum_depth; ++bounce) {
         a.bounce = bounce;
-        switch ((media ? 1 : 0) + (two ? 2 : 0)) {
+        switch ((media ? 1 : 0) + (streamed ? 0 : 2)) {
         case 0: trace_kernel<false, true, false><<<shape.trace_blocks, kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 1: trace_kernel<true, true, false><<<shape.trace_blocks, kStreamBlock, kStreamSharedBytes, stream>>>(a); break;
         case 2: trace_kernel<false, true, true><<<trace_blocks, 128, 0, stream>>>(a); break;
         default: trace_kernel<true, true, true><<<trace_blocks, 128, 0, stream>>>(a); break;
         }
-        if (media && !two) {
+        if (media && streamed) {
             medium_kernel<true><<<shape.shade_blocks, 128, 0, stream>>>(a);
         }
         if (two) {

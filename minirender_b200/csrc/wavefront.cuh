@@ -178,6 +178,17 @@ constexpr uint32_t kSortCells       = 1u << 14;  // >= 2^(3 kSortAxisBits)
 constexpr uint32_t kSortBuckets     = 8u * kSortCells;
 constexpr uint32_t kRaySortMinPaths = 1u << 18;
 constexpr uint32_t kRaySortMinSlots = 4096;
+// Smallest waves (of flattened scenes) whose traversal streams. Streaming pays by refilling lanes: with few rays per
+// lane (the launch has 151,552) its votes and refills cost more than they save. Frames, streamed and
+// not (B200): 262,144 paths: 60k-triangle room 1.65 and 1.62 ms, fogged field 2.53 and 2.36; 480,000:
+// room 1.94 and 1.92; 1,048,576: room 3.52 and 3.78, field 3.24 and 3.37. Scenes of fewer triangle
+// slots than kRaySortMinSlots have rays of a few steps, which refills outweigh longer: 36-triangle
+// box, 1,048,576 paths 1.43 and 1.38 ms, 4,194,304: 4.33 and 4.55.
+constexpr uint32_t kStreamMinPaths        = 1u << 19;
+constexpr uint32_t kStreamMinPathsTrivial = 1u << 21;
+inline bool streams(uint32_t paths, uint32_t slots) {
+    return paths >= (slots < kRaySortMinSlots ? kStreamMinPathsTrivial : kStreamMinPaths);
+}
 // Lanes (workspace + stream) that a plain frame of several waves goes round, so that one wave's
 // last bounces overlap the next waves' first (two lanes: 1M-triangle frame -7.0%; three: a
 // further -1.7%; four: a further -1.0%).
@@ -263,7 +274,7 @@ class Engine {
     // per path. The launch sequence depends only on its arguments, so it can be captured once in
     // a CUDA graph and replayed for every wave of the same depth.
     static void enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, bool media, bool two,
-                                    bool ray_sort, const BatchShape& shape, Workspace& ws,
+                                    bool streamed, bool ray_sort, const BatchShape& shape, Workspace& ws,
                                     cudaStream_t stream);
 
     // Enqueues the per-pixel resolve of a wave's radiance into each job's accumulator and image.
@@ -273,8 +284,8 @@ class Engine {
     static void batch_occupancy(int& trace_blocks_per_sm, int& shade_blocks_per_sm);
 
     // Kernel launches of one wave (paths + resolve).
-    static uint64_t batch_wave_launches(uint32_t maximum_depth, bool media, bool two, bool ray_sort) {
-        return 2ull + (media && !two ? 3ull : 2ull) * (maximum_depth + 1) + (ray_sort ? 4ull * maximum_depth : 0ull);
+    static uint64_t batch_wave_launches(uint32_t maximum_depth, bool media, bool streamed, bool ray_sort) {
+        return 2ull + (media && streamed ? 3ull : 2ull) * (maximum_depth + 1) + (ray_sort ? 4ull * maximum_depth : 0ull);
     }
 };
 

@@ -1,8 +1,8 @@
-"""The streamed traversal (waves of more paths than fit on the device) against the plain one (whole
-paths in one launch): full frames equal the same frame rendered in row bands bit for bit, where each
-frame is large enough to stream and each band small enough not to. Scenes where streaming can go
-wrong: a lone leaf, few triangles, exact distance ties, one-sided surfaces, traversal stacks far
-deeper than their shared part, rays that miss everything, media.
+"""The streamed traversal (waves of many paths) against the plain one: full frames equal the same
+frame rendered in row bands bit for bit, where each frame is large enough to stream, even over a few
+triangles, and each band small enough not to. Scenes where streaming can go wrong: a lone leaf, few
+triangles, exact distance ties, one-sided surfaces, traversal stacks far deeper than their shared
+part, rays that miss everything, media.
 """
 
 import numpy as np
@@ -63,11 +63,11 @@ SCENES = {
 @pytest.mark.parametrize("name", list(SCENES))
 def test_streamed_frame_equals_row_bands(api, name):
     scene = api.Scene(SCENES[name]().snapshot())
-    render = api.RenderSettings(331, 240, 2, 11)  # 158,880 paths: streamed
+    render = api.RenderSettings(331, 240, 27, 11)  # 2,144,880 paths: streamed
     tracer = api.PathTracer(scene, api.IntegratorSettings("mis", 6, True, 3))
     image, counts = tracer.render(render)
     bands, total = [], {k: 0 for k in counts if not k.endswith("tests")}
-    for begin in range(0, 240, 48):  # 31,776 paths a band: one launch each
+    for begin in range(0, 240, 48):  # 428,976 paths a band: not streamed
         band, part = tracer.render_rows(render, begin, begin + 48, statistics=True)
         bands.append(band)
         total = {k: v + part[k] for k, v in total.items()}

@@ -629,7 +629,7 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
                 store_pair(a.st.shadow_o, path, f4(vertex, limit), f4(sd, 0));
                 a.st.shadow_c[path] = f4(beta * ls.radiance * (phase * weight / ls.probability), 0);
                 out.shadow          = true;
-                out.shadow_sort_key = a.q.staging ? coherence_key(s, kNone, vertex, sd) : 0u;
+                out.shadow_sort_key = a.q.shadow_staging ? coherence_key(s, kNone, vertex, sd) : 0u;
             }
         }
         float     pdf;
@@ -706,7 +706,7 @@ __device__ ShadeResult shade_surface(const KernelArgs& a, uint32_t path, int bin
                                                  (weight / ls.probability),
                                              0);
                     out.shadow = true;
-                    out.shadow_sort_key = a.q.staging ? coherence_key(s, slot, origin, sd) : 0u;
+                    out.shadow_sort_key = a.q.shadow_staging ? coherence_key(s, slot, origin, sd) : 0u;
                 }
             }
         }
@@ -773,9 +773,9 @@ __global__ void __launch_bounds__(128, 5) shade_kernel(KernelArgs a) {
             sort_key             = r.continue_path ? r.sort_key : kNone;
             shadow_sort          = r.shadow ? r.shadow_sort_key : kNone;
         }
-        if (a.q.staging) {
-            // Both queues are staged for the coherence sort: each entry's key beside it, one
-            // count per distinct key per warp (shadow keys in the second half of the counts).
+        // A queue that the coherence sort orders is staged: each entry's key beside it, one count
+        // per distinct key per warp (shadow keys in the second half of the counts).
+        if (a.q.shadow_staging) {
             const uint32_t pos = warp_append(shadow_key, path, &ctr->shadow, a.q.shadow_staging, 0);
             if (shadow_key != kNone) {
                 a.q.shadow_keys[pos] = shadow_sort;
@@ -952,7 +952,7 @@ __host__ void enqueue_sort_scan(uint32_t* buckets, cudaStream_t stream) {
 // path results do not depend on queue order).
 __global__ void sort_scatter_kernel(KernelArgs a) {
     const uint32_t n_ext    = a.q.counters[a.bounce + 1].ext;
-    const uint32_t n_shadow = a.q.counters[a.bounce].shadow;
+    const uint32_t n_shadow = a.q.shadow_staging ? a.q.counters[a.bounce].shadow : 0u;
     const uint32_t n        = n_ext + n_shadow;
     uint32_t*      next     = a.q.ext[(a.bounce + 1) & 1];
     const uint32_t step     = gridDim.x * blockDim.x;
@@ -1381,7 +1381,7 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
     const int          variant = (media ? 1 : 0) + (two ? 2 : 0);
     // Kernel timing counts the wavefront's traversal launches, and the shadow capture reads its queue.
     if (init.count <= shape.path_lanes[variant] && !init.capture && !kernel_timing().enabled.load()) {
-        a.q.staging = nullptr;  // no sort keys
+        a.q.staging = a.q.shadow_staging = nullptr;  // no sort keys
         switch (variant) {
         case 0: path_kernel<false, false><<<blocks, 128, 0, stream>>>(a, init.count); break;
         case 1: path_kernel<true, false><<<blocks, 128, 0, stream>>>(a, init.count); break;
@@ -1398,12 +1398,15 @@ void Engine::run_wave(const Scene& scene, const IntegratorParams& params, const 
     if (!ray_sort) {
         a.q.staging = nullptr;
     }
-    KernelTiming&      timing = kernel_timing();
-    bool               timed  = false;
-    timed = timing.enabled.load();
     // Waves of few rays per lane do not stream (see kStreamMinPaths): the two-level scenes' kernel
     // traces them too.
     const bool streamed = !two && streams(init.count, scene.d.slot_count);
+    if (!ray_sort || (media && streamed)) {
+        a.q.shadow_staging = nullptr;  // see Queues
+    }
+    KernelTiming&      timing = kernel_timing();
+    bool               timed  = false;
+    timed = timing.enabled.load();
     const int  traced   = (media ? 1 : 0) + (streamed ? 0 : 2);
     note_launches(1 + (media && streamed ? 3ull : 2ull) * (params.maximum_depth + 1) + (ray_sort ? 4ull * params.maximum_depth : 0ull) +
                   (init.capture ? 1 : 0));
@@ -1504,6 +1507,9 @@ void Engine::enqueue_batch_paths(const WaveDesc* wave, uint32_t maximum_depth, b
     ray_sort       = ray_sort && ws.queues.staging != nullptr;
     if (!ray_sort) {
         a.q.staging = nullptr;
+    }
+    if (!ray_sort || (media && streamed)) {
+        a.q.shadow_staging = nullptr;  // see Queues
     }
     // The variants that do not stream keep fewer blocks resident (more registers per thread): their
     // grid is capped at what fits, the persistent loop takes the work either way.

@@ -33,6 +33,7 @@ struct mr_scene {
 namespace mr {
 
 void copy_path_radiance(Workspace& ws, uint32_t count, float* device_out, cudaStream_t stream);
+void load_path_kernels();
 void set_last_error(const std::string& message);
 
 namespace {
@@ -56,6 +57,9 @@ static __device__ __align__(256) unsigned char g_trace_scratch[kScratchBytes];
 std::mutex                   setup_mutex;
 std::array<unsigned char*, 64> scratch_address{};
 
+__global__ void stage_rays_kernel(const mr_ray* rays, uint32_t count, float4* staging, unsigned* invalid);
+__global__ void check_output_kernel(const float* radiance, uint32_t count, unsigned* error);
+
 unsigned char* device_scratch() {
     int device = 0;
     MR_CUDA(cudaGetDevice(&device));
@@ -64,6 +68,11 @@ unsigned char* device_scratch() {
     if (!scratch_address[device]) {
         void* ptr = nullptr;
         MR_CUDA(cudaGetSymbolAddress(&ptr, g_trace_scratch));
+        // The kernels of a call are loaded here too, so that no later call places code.
+        cudaFuncAttributes attributes;
+        MR_CUDA(cudaFuncGetAttributes(&attributes, stage_rays_kernel));
+        MR_CUDA(cudaFuncGetAttributes(&attributes, check_output_kernel));
+        load_path_kernels();
         scratch_address[device] = static_cast<unsigned char*>(ptr);
     }
     return scratch_address[device];

@@ -455,8 +455,8 @@ mr_status mr_capture_shadow_rays(const mr_scene* scene, const mr_integrator_sett
  * `stream` is a cudaStream_t (null = legacy default stream); the call returns after the work
  * has finished. The working memory is one fixed array of about 4.3 MB inside the library, held
  * on every GPU that loads it until the process exits. The first call on a device looks up the
- * array's address, which under CUDA's lazy module loading also loads the module and places the
- * array in device memory (an allocation and a synchronisation): warm up each device with a call
+ * array's address and loads the call's kernels, which under CUDA's lazy module loading places the
+ * array and their code in device memory (an allocation and a synchronisation): warm up each device with a call
  * of count 0 (null buffers allowed) before any stream capture and before the phase that must not
  * allocate. The address is cached per device and must not be used across a cudaDeviceReset.
  * Calls share that array: it is cleared at the start of each call, and calls whose GPU work

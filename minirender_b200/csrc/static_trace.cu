@@ -10,8 +10,8 @@
 // process exits). Inputs and outputs stay in the caller's device memory.
 //
 // The array's device address is resolved once per device with cudaGetSymbolAddress (the name in
-// host code is only a host-side stand-in). The first call on a device does this, and with CUDA's
-// lazy module loading that lookup is also what loads the module and places the array in device
+// host code is only a host-side stand-in). The first call on a device does this and loads the
+// call's kernels, which with CUDA's lazy module loading places the array and their code in device
 // memory (which can allocate and synchronise): make that first call a zero-length one (count 0),
 // before any stream capture and before the caller's no-allocation phase. The cached address
 // belongs to the device's primary context: the entry point must not be used across a

@@ -1231,7 +1231,12 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
     ws->queues.shadow_staging = reinterpret_cast<uint32_t*>(base + o_sstage);
     ws->queues.shadow_keys    = reinterpret_cast<uint32_t*>(base + o_skeys);
     ws->queues.buckets      = reinterpret_cast<uint32_t*>(base + o_buck);
-    MR_CUDA(cudaMemset(ws->queues.buckets, 0, 2 * kSortBuckets * sizeof(uint32_t)));
+    // Cleared before the workspace is handed out: its user's stream is a non-blocking one, which the
+    // legacy stream's work is not ordered before (a clear there would wait behind whatever the caller
+    // has queued on it, while a wave counts into memory that nobody has written).
+    CallStream clear;
+    MR_CUDA(cudaMemsetAsync(ws->queues.buckets, 0, 2 * kSortBuckets * sizeof(uint32_t), clear.stream));
+    MR_CUDA(cudaStreamSynchronize(clear.stream));
     ws->queues.counters     = reinterpret_cast<BounceCounters*>(base + o_ctr);
     ws->queues.set_statistics(base + o_stats);
     ws->accumulator         = reinterpret_cast<float4*>(base + o_acc);

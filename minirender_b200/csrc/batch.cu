@@ -208,7 +208,9 @@ class Server {
         }
         stages_ = kAheadPerLane * b.concurrent_waves + 1;
         MR_CUDA(cudaMalloc(&d_errors_, settings_.max_jobs * sizeof(unsigned)));
-        MR_CUDA(cudaMemset(d_errors_, 0, settings_.max_jobs * sizeof(unsigned)));
+        // On the server's own stream: the lanes' streams are not ordered after the legacy one.
+        MR_CUDA(cudaMemsetAsync(d_errors_, 0, settings_.max_jobs * sizeof(unsigned), stream_));
+        MR_CUDA(cudaStreamSynchronize(stream_));
         stage_.assign(stages_, nullptr);
         h_errors_.assign(stages_, nullptr);
         for (uint32_t k = 0; k < stages_; ++k) {

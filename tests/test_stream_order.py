@@ -11,7 +11,7 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "minirender_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["wavefront.cu"])
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
 def test_no_clear_on_the_legacy_stream(name):
     with open(os.path.join(CSRC, name)) as f:
         source = f.read()

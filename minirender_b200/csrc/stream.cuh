@@ -93,15 +93,22 @@ struct StreamStack {
 
 // The local part of a lane's stack: the moved entries, their count in the first element. spill()
 // and restore() take and return `top` by value and are not inlined, so the hot loop keeps the stack
-// in registers.
-constexpr int kDeepSize = 1 + kStackSize;
+// in registers. Each spill but the first moves the mark of the one before along with kMoved - 1 nodes,
+// and the shared part holds kFull - 2 nodes beside the end mark and the newest mark, so kSpills spills
+// hold kStackSize nodes.
+constexpr uint32_t kSpillNodes = StreamStack::kMoved - 1;
+constexpr uint32_t kSpills =
+    (kStackSize - 1 - (StreamStack::kFull - 2) + kSpillNodes - 1) / kSpillNodes;
+constexpr uint32_t kDeepNodes = kSpills * StreamStack::kMoved;
+constexpr uint32_t kDeepSize  = 1 + kDeepNodes;
+static_assert(1 + kSpills * kSpillNodes + StreamStack::kFull - 2 >= kStackSize, "spilled nodes and shared ones");
 
 // For a full() stack: entries kMark .. kMark + kMoved - 1 move, the newer ones close up. Returns the
 // new top, 0 when the local part is full too.
 static __device__ __noinline__ uint32_t spill(uint32_t base, uint32_t top, int2* deep) {
     constexpr uint32_t step = StreamStack::kStep;
     const uint32_t     moved = static_cast<uint32_t>(deep[0].x);
-    if (moved + StreamStack::kMoved > kStackSize) {
+    if (moved + StreamStack::kMoved > kDeepNodes) {
         return 0;
     }
     const uint32_t mark = base + StreamStack::kMark * step;
@@ -258,7 +265,8 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
                 stack.push(v.r2, v.t2);
                 stack.push(v.r1, v.t1);
                 // Every visit counts and each leaf was pushed by one, so this ends traversal on any
-                // tree; the stack holds what an accepted tree can need.
+                // tree; the stack, with its local part, holds the kStackSize nodes that cover every
+                // accepted tree.
                 ray.word += 1u << 16;
                 if (ray.word >= 0xffff0000u || stack.full()) {
                     const bool visits = ray.word >= 0xffff0000u;

@@ -141,7 +141,10 @@ struct StreamRay {
     f3       o;
     float    inv_lo[3], inv_hi[3];
     float    sx, sy, sz;
-    uint32_t word;  // bits 0-3 near_xy, 4-7 near_z, 8-13 kx ky kz, 16-31 visits
+    uint32_t word;  // bits 0-3 near_xy, 4-7 near_z, 8-13 kx ky kz, 14-31 visits
+    static constexpr uint32_t kVisit    = 1u << 14;
+    static constexpr uint32_t kTooMany  = (kMaxVisits + 1) * kVisit;  // a word that counts more than kMaxVisits
+    static_assert(kMaxVisits + 1 < 1u << 18, "the count's bits");
     __device__ __forceinline__ void init(const RayQuery& q) {
         o = q.o;
         for (int a = 0; a < 3; ++a) {
@@ -180,7 +183,7 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
     int            node = kNoNode, leaf = 0;
     float          tmin = 0;
     NearestHit     hit{0, kNone};
-    StreamRay      ray;
+    StreamRay      ray{};
     uint32_t       next = 0, end = 0;  // the rest of the warp's chunk
     int            refill = kRefill;  // 32 once the queue is empty
     int2           deep[kDeepSize];
@@ -191,6 +194,7 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
         if (node < 0 && leaf == 0) {  // postpone the first leaf and keep descending
             leaf = node;
             node = kPopNode;
+            ray.word += StreamRay::kVisit;
         }
         const bool     idle      = node >= kDeepNode && leaf == 0;  // finished, or waiting for restore()
         const bool     interior  = static_cast<unsigned>(node) < static_cast<unsigned>(kPopNode);
@@ -199,6 +203,9 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
         const unsigned idles     = __ballot_sync(0xffffffffu, idle);
         if (__popc(idles) >= refill) {
             const bool done = idle && node == kNoNode;
+            if (done && filled && ray.word >= StreamRay::kTooMany) {  // with its last leaves
+                io.fail(kErrorVisits);
+            }
             io.finish(done && filled, ray, hit);
             filled = filled && !done;
             if (idle && !done) {
@@ -267,9 +274,9 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
                 // Every visit counts and each leaf was pushed by one, so this ends traversal on any
                 // tree; the stack, with its local part, holds the kStackSize nodes that cover every
                 // accepted tree.
-                ray.word += 1u << 16;
-                if (ray.word >= 0xffff0000u || stack.full()) {
-                    const bool visits = ray.word >= 0xffff0000u;
+                ray.word += StreamRay::kVisit;
+                if (ray.word >= StreamRay::kTooMany || stack.full()) {
+                    const bool visits = ray.word >= StreamRay::kTooMany;
                     stack.top         = visits ? 0 : spill(stack.base, stack.top, deep);
                     if (stack.top == 0) {
                         io.fail(visits ? kErrorVisits : kErrorStack);

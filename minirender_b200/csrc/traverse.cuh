@@ -19,7 +19,7 @@ namespace mr {
 // bvh.cpp:16; imported trees are refused beyond 64 levels), so at most 3 * 63 entries are
 // stacked before any push: the check `sp > kStackSize - 3` never fires on an accepted tree.
 constexpr int      kStackSize  = 195;
-constexpr uint32_t kMaxVisits  = 1u << 16;  // node visits per ray before the query gives up
+constexpr uint32_t kMaxVisits  = 1u << 16;  // node visits and leaves per ray before the query gives up
 
 // The part of a ray that the triangle test uses: origin, permutation and shear.
 struct TriangleRay {
@@ -272,8 +272,7 @@ constexpr int kPopNode  = 0x7ffffffd;  // stream.cuh: the next node is on the st
 // What bounds it is the load-store pipe (one wavefront per divergent lane and load) and issue
 // slots, so a node visit is four 32-byte loads and packed arithmetic, and the state kept across
 // the loops is what the loops use: the hit is a distance and a slot, `direction()` fetches the
-// ray's direction again for the rare single-sided triangle, and the visit bound is the box-test
-// count.
+// ray's direction again for the rare single-sided triangle.
 template <bool ANY_HIT, typename Direction>
 __device__ __forceinline__ NearestHit trace(const DeviceScene& s, const RayQuery& q, float tmin, float tmax,
                                             Direction direction, TraceCounters& counters, unsigned& error) {
@@ -302,9 +301,9 @@ __device__ __forceinline__ NearestHit trace(const DeviceScene& s, const RayQuery
     const f3    neg_o = -q.o;
     SectorOffsets at;
     at.init(q.neg);
-    // Every node visit counts at least two box tests and each leaf reference was pushed by a
-    // visit, so bounding the count ends traversal on any tree.
-    const uint32_t bounds_limit = counters.bounds + 2 * kMaxVisits;
+    // Every pass of every loop below visits a node or tests a leaf, and both count against
+    // kMaxVisits, so traversal ends on any tree; the streamed walk counts the same.
+    uint32_t visits = 0;
     // Next stacked subtree that can still contain a nearer hit, or kNoNode.
     const auto pop = [&]() {
         while (sp > 0) {
@@ -324,14 +323,14 @@ __device__ __forceinline__ NearestHit trace(const DeviceScene& s, const RayQuery
         }
         // Interior phase.
         while (alive && node >= 0) {
+            if (++visits > kMaxVisits) {
+                error |= kErrorVisits;
+                return result;
+            }
             NodeVisit v;
             v.visit(s.nodes + kWideNode * static_cast<size_t>(node), at, neg_o, neg_o, q.inv_lo, q.inv_hi, tmin,
                     result.t);
             counters.bounds += v.children();
-            if (counters.bounds > bounds_limit) {
-                error |= kErrorVisits;
-                return result;
-            }
             v.sort();
             if (v.t0 != inf) {
                 if (sp > kStackSize - 3) {
@@ -362,6 +361,10 @@ __device__ __forceinline__ NearestHit trace(const DeviceScene& s, const RayQuery
         }
         // Leaf phase: the postponed leaf, then any leaf the lane now points at.
         while (held) {
+            if (++visits > kMaxVisits) {
+                error |= kErrorVisits;
+                return result;
+            }
             for (uint32_t slot = static_cast<uint32_t>(~leaf);; ++slot) {
                 const float4* tp = s.tris + 3 * static_cast<size_t>(slot);
                 const float4  a4 = __ldg(tp + 0);

@@ -113,3 +113,64 @@ def test_deepest_tree_fits_the_stacks(api, hit, paths):
     tracer = api.PathTracer(scene, api.IntegratorSettings("mis", 1, True, 3))
     radiance, _ = tracer.trace(o, d, 0.0, np.inf, keys)
     np.testing.assert_array_equal(radiance, np.where(along, 0, np.float32(0.5))[:, None].repeat(3, 1))
+
+
+LIMIT = 65536  # node visits and leaves of one ray
+
+
+def beads(levels, decoys):
+    """A tree whose 2^levels - 1 wide nodes the +z axis enters one after the other, each with two
+    children of its own beside the axis (four at the bottom), and no triangle. `decoys` bottom leaves
+    have boxes that the axis enters: node visits and leaves of an axis ray are 2^levels - 1 + decoys."""
+    near = np.array([(4, -0.5), (5, -0.5), (4, 0.5)], float)
+    passed = np.array([(-0.4, -0.5), (0.5, -0.5), (0.5, 0.4)], float)
+    triangles, left = [], decoys
+
+    def triangle(side):
+        xy = passed if side == 0 else near * (side, 1)
+        triangles.append(np.column_stack([xy, np.full(3, len(triangles) + 1.0)]))
+        return len(triangles) - 1
+
+    def node(level):
+        nonlocal left
+        if level == 1:
+            left, decoy = max(0, left - 1), left > 0
+            return (triangle(1), triangle(-1)), (triangle(1), triangle(0 if decoy else -1))
+        first = node(level - 1), triangle(1)
+        return first, (node(level - 1), triangle(-1))
+
+    tree = node(levels)
+    return np.array(triangles), tree
+
+
+@pytest.fixture(scope="module")
+def bead_scenes(api):
+    return {decoys: imported(api, *beads(16, decoys)) for decoys in (1, 2)}
+
+
+@pytest.mark.parametrize("decoys", [1, 2])
+@pytest.mark.parametrize("paths", [None, 1 << 10, 1 << 19], ids=["query", "few", "streamed"])
+def test_visit_bound_is_the_same_on_every_route(api, bead_scenes, paths, decoys):
+    scene = bead_scenes[decoys]
+    accepted = (1 << 16) - 1 + decoys <= LIMIT
+    o, d, keys, along = axis_rays(paths or 64, 64)
+    tracer = api.PathTracer(scene, api.IntegratorSettings("mis", 1, True, 3))
+
+    def calls():
+        if paths is None:
+            yield lambda: scene.intersect(o, d, 0.0, np.inf)
+            yield lambda: scene.occluded(o, d, 0.0, np.inf)
+        else:
+            yield lambda: tracer.trace(o, d, 0.0, np.inf, keys)
+
+    for call in calls():
+        if not accepted:
+            with pytest.raises(api.MiniRenderError, match="node-visit bound"):
+                call()
+            continue
+        out, counts = call()
+        if paths is None:
+            assert counts["bounds_tests"] == 64 * (1 + 4 * ((1 << 16) - 1)) and counts["triangle_tests"] == 64
+            assert not (out if out.dtype == bool else out["primitive"] != 0xffffffff).any()
+        else:
+            np.testing.assert_array_equal(out, np.full((paths, 3), 0.5, np.float32))

@@ -222,9 +222,12 @@ __device__ __forceinline__ bool triangle_test(const TriangleRay& q, f3 v0, f3 v1
     const float edge       = fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c));
     const float error = 3.0f * (g3 * edge * z + error_edge * z + g3 * z * edge);
     // distance <= error / |determinant|, with the division only where the products are within
-    // 2^-20 of each other (or not finite): elsewhere their rounding cannot change the answer.
+    // 2^-20 of each other (or not finite, or where the product or the distance is near or below the
+    // normal range, so that the quotient may be subnormal and round up by more): elsewhere their
+    // rounding cannot change the answer.
     const float scaled = distance * fabsf(determinant);
-    if (!(scaled > error * 1.00000095367431640625f && scaled < __int_as_float(0x7f800000) && scaled > 1e-30f)) {
+    if (!(scaled > error * 1.00000095367431640625f && scaled < __int_as_float(0x7f800000) && scaled > 1e-30f &&
+          distance >= kFltMin)) {
         if (distance <= error / fabsf(determinant)) {
             return false;
         }

@@ -201,13 +201,13 @@ class Server {
             MR_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
             MR_CUDA(cudaEventCreateWithFlags(&lane.mark, cudaEventDisableTiming));
             lane.ws = acquire_workspace(b.wave_paths, kMaxDepth + 1, 0);
-            MR_CUDA(cudaMalloc(&lane.d_wave, sizeof(WaveDesc)));
+            MR_CUDA(allocate_device([&] { return cudaMalloc(&lane.d_wave, sizeof(WaveDesc)); }));
             MR_CUDA(cudaMemsetAsync(lane.ws->queues.stats, 0, kStatCount * sizeof(unsigned long long),
                                     lane.stream));
             MR_CUDA(cudaStreamSynchronize(lane.stream));
         }
         stages_ = kAheadPerLane * b.concurrent_waves + 1;
-        MR_CUDA(cudaMalloc(&d_errors_, settings_.max_jobs * sizeof(unsigned)));
+        MR_CUDA(allocate_device([&] { return cudaMalloc(&d_errors_, settings_.max_jobs * sizeof(unsigned)); }));
         // On the server's own stream: the lanes' streams are not ordered after the legacy one.
         MR_CUDA(cudaMemsetAsync(d_errors_, 0, settings_.max_jobs * sizeof(unsigned), stream_));
         MR_CUDA(cudaStreamSynchronize(stream_));
@@ -431,8 +431,9 @@ class Server {
         DeviceGuard guard(device_);
         admin_after_lanes();
         float* d = nullptr;
-        MR_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d), 3 * j.pixels * sizeof(float), pool_,
-                                        stream_));
+        MR_CUDA(allocate_device([&] {
+            return cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d), 3 * j.pixels * sizeof(float), pool_, stream_);
+        }));
         preview_kernel<<<static_cast<unsigned>((j.pixels + 255) / 256), 256, 0, stream_>>>(
             j.accumulator, j.width, j.pixels, j.issued.sample, j.issued.row, d);
         MR_CUDA(cudaGetLastError());
@@ -592,8 +593,11 @@ class Server {
             queued_.pop_front();
             void* acc = nullptr;
             void* rgb = nullptr;
-            if (cudaMallocFromPoolAsync(&acc, j.pixels * 2 * sizeof(float4), pool_, stream_) != cudaSuccess ||
-                cudaMallocFromPoolAsync(&rgb, j.pixels * 3 * sizeof(float), pool_, stream_) != cudaSuccess) {
+            const auto allocate = [&](void** p, size_t bytes) {
+                return allocate_device([&] { return cudaMallocFromPoolAsync(p, bytes, pool_, stream_); });
+            };
+            if (allocate(&acc, j.pixels * 2 * sizeof(float4)) != cudaSuccess ||
+                allocate(&rgb, j.pixels * 3 * sizeof(float)) != cudaSuccess) {
                 cudaGetLastError();
                 if (acc) {
                     cudaFreeAsync(acc, stream_);

@@ -14,6 +14,22 @@ namespace mr {
 // keeps up to 2 GB of freed memory for reuse).
 cudaMemPool_t library_pool();
 
+// Frees the idle pooled workspaces of the current device (wavefront.cu); false when there are none.
+bool drop_pooled_workspaces();
+
+// Makes a device allocation; where that fails for lack of memory, once more without the idle pooled
+// workspaces. A failed allocation is not a sticky error and is not left for the next call to find.
+template <typename Allocation> cudaError_t allocate_device(Allocation&& allocation) {
+    cudaError_t e = allocation();
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        if (drop_pooled_workspaces() && (e = allocation()) == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+        }
+    }
+    return e;
+}
+
 // A non-blocking stream of the current device for the length of a call. Streams are pooled per
 // process (creating and destroying one takes 150-300 us, most of a small call): a call returns its
 // stream with its work done or ordered on it, and at most kPooledStreams wait for the next calls.
@@ -91,12 +107,14 @@ template <typename T> struct DeviceBuffer {
         if (n == 0) {
             return;
         }
+        void** at = reinterpret_cast<void**>(&ptr);
         if (AllocationScope::current_id != 0) {
-            MR_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ptr), n * sizeof(T), library_pool(),
-                                            AllocationScope::current));
+            MR_CUDA(allocate_device([&] {
+                return cudaMallocFromPoolAsync(at, n * sizeof(T), library_pool(), AllocationScope::current);
+            }));
             scope = AllocationScope::current_id;
         } else {
-            MR_CUDA(cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T)));
+            MR_CUDA(allocate_device([&] { return cudaMalloc(at, n * sizeof(T)); }));
         }
         count = n;
     }

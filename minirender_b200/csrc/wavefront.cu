@@ -1179,13 +1179,6 @@ std::vector<std::shared_ptr<Workspace>> pool;  // least recently used first
 constexpr size_t kPooledWorkspaces     = 16;
 constexpr size_t kPooledWorkspaceBytes = size_t(12) << 30;  // four lanes of 8M paths and some small ones
 
-void drop_pooled_workspaces() {
-    std::vector<std::shared_ptr<Workspace>> dropped;
-    std::lock_guard<std::mutex>             lock(pool_mutex);
-    dropped.swap(pool);
-}
-
-
 std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     auto   ws     = std::make_shared<Workspace>();
     size_t offset = 0;
@@ -1209,11 +1202,7 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
     const size_t o_stats = field(kStatisticsBytes);
     const size_t o_acc = field(2 * pixels * sizeof(float4));
     void*        mem   = nullptr;
-    if (cudaMalloc(&mem, offset) == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();  // not a sticky error: pooled workspaces may make room
-        drop_pooled_workspaces();
-        MR_CUDA(cudaMalloc(&mem, offset));
-    }
+    MR_CUDA(allocate_device([&] { return cudaMalloc(&mem, offset); }));
     char* base              = static_cast<char*>(mem);
     ws->memory              = mem;
     ws->bytes               = offset;
@@ -1250,7 +1239,7 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
 // a multiple of 16) so that one workspace serves many job shapes. Above kPooledWorkspaces or
 // kPooledWorkspaceBytes the least recently used go (when the smallest went, a shape that a few
 // larger ones did not cover was allocated and freed on every call: 3.6 ms of a 22 ms frame), and
-// all of them go when an allocation fails.
+// all of a device's go when any of the library's allocations there fails (allocate_device).
 std::shared_ptr<Workspace> acquire_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     int device = 0;
     MR_CUDA(cudaGetDevice(&device));
@@ -1283,6 +1272,18 @@ std::shared_ptr<Workspace> acquire_workspace(size_t capacity, uint32_t max_bounc
     auto ws    = allocate_workspace(capacity, max_bounces, pixels);
     ws->device = device;
     return ws;
+}
+
+bool drop_pooled_workspaces() {
+    int device = 0;
+    MR_CUDA(cudaGetDevice(&device));
+    std::vector<std::shared_ptr<Workspace>> dropped;  // freed (a device-wide wait) outside the lock
+    std::lock_guard<std::mutex>             lock(pool_mutex);
+    const auto idle = std::stable_partition(pool.begin(), pool.end(),
+                                            [&](const auto& w) { return w->device != device; });
+    dropped.assign(std::make_move_iterator(idle), std::make_move_iterator(pool.end()));
+    pool.erase(idle, pool.end());
+    return !dropped.empty();
 }
 
 void release_workspace(std::shared_ptr<Workspace> ws) {

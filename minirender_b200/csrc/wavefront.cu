@@ -1176,8 +1176,12 @@ namespace {
 std::mutex                              pool_mutex;
 std::vector<std::shared_ptr<Workspace>> pool;  // least recently used first
 
+// Limits of the pool, per device: kKeptWorkspaces of any size (a frame's or a batch's lanes, however
+// large their waves), more of them up to kPooledWorkspaces and kPooledWorkspaceBytes (four lanes of 8M
+// paths and some small ones).
+constexpr size_t kKeptWorkspaces       = 4;
 constexpr size_t kPooledWorkspaces     = 16;
-constexpr size_t kPooledWorkspaceBytes = size_t(12) << 30;  // four lanes of 8M paths and some small ones
+constexpr size_t kPooledWorkspaceBytes = size_t(12) << 30;
 
 std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     auto   ws     = std::make_shared<Workspace>();
@@ -1236,10 +1240,9 @@ std::shared_ptr<Workspace> allocate_workspace(size_t capacity, uint32_t max_boun
 
 // Workspaces are pooled per process: a request takes the smallest pooled workspace of its device
 // that is large enough in every dimension, and requests are rounded up (powers of two, bounces to
-// a multiple of 16) so that one workspace serves many job shapes. Above kPooledWorkspaces or
-// kPooledWorkspaceBytes the least recently used go (when the smallest went, a shape that a few
-// larger ones did not cover was allocated and freed on every call: 3.6 ms of a 22 ms frame), and
-// all of a device's go when any of the library's allocations there fails (allocate_device).
+// a multiple of 16) so that one workspace serves many job shapes. Above the pool's limits a device's
+// least recently used go (when the smallest went, a shape that a few larger ones did not cover was
+// allocated and freed on every call: 3.6 ms of a 22 ms frame), and all of a device's go when any of the library's allocations there fails (allocate_device).
 std::shared_ptr<Workspace> acquire_workspace(size_t capacity, uint32_t max_bounces, size_t pixels) {
     int device = 0;
     MR_CUDA(cudaGetDevice(&device));
@@ -1290,17 +1293,24 @@ void release_workspace(std::shared_ptr<Workspace> ws) {
     if (!ws) {
         return;
     }
+    const int                               device = ws->device;
     std::vector<std::shared_ptr<Workspace>> dropped;  // freed (a device-wide wait) outside the lock
     std::lock_guard<std::mutex>             lock(pool_mutex);
     pool.push_back(std::move(ws));
-    size_t bytes = 0;
+    size_t bytes = 0, count = 0;
     for (const auto& w : pool) {
-        bytes += w->bytes;
+        if (w->device == device) {
+            bytes += w->bytes;
+            ++count;
+        }
     }
-    while (pool.size() > 1 && (pool.size() > kPooledWorkspaces || bytes > kPooledWorkspaceBytes)) {
-        bytes -= pool.front()->bytes;
-        dropped.push_back(std::move(pool.front()));
-        pool.erase(pool.begin());
+    while (count > kPooledWorkspaces || (count > kKeptWorkspaces && bytes > kPooledWorkspaceBytes)) {
+        const auto oldest =
+            std::find_if(pool.begin(), pool.end(), [&](const auto& w) { return w->device == device; });
+        bytes -= (*oldest)->bytes;
+        --count;
+        dropped.push_back(std::move(*oldest));
+        pool.erase(oldest);
     }
 }
 

@@ -1,4 +1,6 @@
-"""Idle pooled workspaces give way to any other allocation of the library."""
+"""Idle pooled workspaces give way to any other allocation of the library, and the workspaces of a
+batch's lanes stay pooled when a batch of another shape follows, however large their waves.
+"""
 
 import os
 import subprocess
@@ -64,3 +66,23 @@ with api.RenderServer(1 << 30, batch=api.BatchSettings(wave_paths=1 << 16, concu
 @pytest.mark.parametrize("call", list(CALLS))
 def test_allocations_take_the_place_of_idle_workspaces(call):
     run(FULL % CALLS[call])
+
+
+LARGE_LANES = """
+import torch
+from minirender_b200 import api, scene as sc
+scene = api.Scene(sc.job_scene(500, 5).snapshot())
+jobs = [api.BatchJob(scene, api.RenderSettings(64, 64, 2, 1), api.IntegratorSettings("mis", 2, True, 3))]
+small, large = (api.BatchSettings(wave_paths=1 << k, concurrent_waves=4) for k in (16, 24))
+assert api.render_batch(jobs, small)[1] == [0]  # loads the kernels
+free = torch.cuda.mem_get_info()[0]
+for lanes in (large, small, large, small):  # a batch of another shape gives the lanes' workspaces back
+    assert api.render_batch(jobs, lanes)[1] == [0]
+    # Four workspaces of 2^24 paths, of more than 192 bytes each (a path's records).
+    assert free - torch.cuda.mem_get_info()[0] > 4 * 192 * (1 << 24)
+print("done")
+"""
+
+
+def test_lanes_of_large_waves_stay_pooled():
+    run(LARGE_LANES)

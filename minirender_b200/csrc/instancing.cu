@@ -382,7 +382,7 @@ void build_mesh_trees(Scene& scene, const mr_scene_desc& desc, cudaStream_t stre
         mt.node_count = built.node_count;
         mt.leaves     = built.leaves;
         mt.depth      = built.maximum_depth;
-        wides[m]      = collapse_tree(mt.nodes.ptr, mt.node_count, stream);
+        wides[m]      = collapse_tree(mt.nodes.ptr, built_interior(mt.node_count), stream);
         mt.wide_children = std::move(wides[m].children);
         mt.node_base  = node_total;
         mt.wide_count = wides[m].count;
@@ -487,7 +487,7 @@ void build_instance_tree(Scene& scene, cudaStream_t stream) {
     MR_CUDA(cudaGetLastError());
     BuildResult built = build_bvh_device(lo.ptr, hi.ptr, centroid.ptr, count, stream);
     scene.build_seconds += built.seconds;
-    WideTree wide       = collapse_tree(built.nodes.ptr, built.node_count, stream);
+    WideTree wide       = collapse_tree(built.nodes.ptr, built_interior(built.node_count), stream);
     t.tlas_nodes        = std::move(wide.nodes);
     t.tlas_node_count   = built.node_count;
     t.tlas_depth        = built.maximum_depth;

@@ -107,6 +107,9 @@ __device__ __forceinline__ float node_area(const mr_bvh_node& n) {
     return ex * ey + ey * ez + ez * ex;
 }
 
+// Most interior nodes of an imported tree: wide nodes have nonnegative int indices.
+constexpr uint64_t kMaxInterior = 0x3fffffff;
+
 // A level of the collapse: how many wide nodes it has and the index of its first.
 struct CollapseLevel {
     uint32_t count, base;
@@ -191,14 +194,6 @@ __global__ void collapse_write_kernel(const mr_bvh_node* nodes, const int4* all_
     float4* o = wide + kWideNode * (static_cast<size_t>(base) + k);
     write_wide_boxes(o, lo, hi);
     write_wide_refs(o, ref);
-}
-
-__global__ void interior_count_kernel(const mr_bvh_node* nodes, uint32_t count, uint32_t* total) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned m = __ballot_sync(0xffffffffu, i < count && nodes[i].count == 0);
-    if ((threadIdx.x & 31) == 0 && m) {
-        atomicAdd(total, static_cast<uint32_t>(__popc(m)));
-    }
 }
 
 // Triangle stream in leaf order; marks the last slot of every leaf.
@@ -369,19 +364,10 @@ float determinant3(const float* m) {
            e(2, 0) * (e(0, 1) * e(1, 2) - e(1, 1) * e(0, 2));
 }
 
-WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t node_count, cudaStream_t stream) {
-    WideTree out;
-    if (node_count == 0) {
-        return out;
-    }
+WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t interior, cudaStream_t stream) {
+    WideTree    out;
     mr_bvh_node root{};
     MR_CUDA(cudaMemcpyAsync(&root, ref_nodes, sizeof(root), cudaMemcpyDeviceToHost, stream));
-    DeviceBuffer<uint32_t> total;
-    total.allocate(1);
-    MR_CUDA(cudaMemsetAsync(total.ptr, 0, sizeof(uint32_t), stream));
-    interior_count_kernel<<<(node_count + 255) / 256, 256, 0, stream>>>(ref_nodes, node_count, total.ptr);
-    uint32_t interior = 0;
-    MR_CUDA(cudaMemcpyAsync(&interior, total.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
     MR_CUDA(cudaStreamSynchronize(stream));
     for (int a = 0; a < 3; ++a) {
         out.lo[a] = root.minimum[a];
@@ -820,7 +806,7 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
         // ---- BVH (reference layout on the device) ----
         DeviceBuffer<mr_bvh_node> ref_nodes;
         DeviceBuffer<uint32_t>    ref_order;
-        uint32_t                  node_count = 0;
+        uint32_t                  node_count = 0, interior = 0;
         if (prims) {
             if (bvh) {
                 node_count = bvh->node_count;
@@ -832,7 +818,7 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
                                         cudaMemcpyHostToDevice, stream));
                 // Statistics of the imported tree (host walk).
                 std::vector<std::pair<uint32_t, uint32_t>> stack{{0u, 0u}};
-                uint64_t leaves = 0, depth = 0;
+                uint64_t leaves = 0, depth = 0, inner = 0;
                 while (!stack.empty()) {
                     const auto [i, d] = stack.back();
                     stack.pop_back();
@@ -842,12 +828,14 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
                         ++leaves;
                     } else {
                         require(d < 64, "Imported BVH is deeper than 64 levels");
+                        require(++inner <= kMaxInterior, "Imported BVH has too many nodes");
                         stack.push_back({n.first, d + 1});
                         stack.push_back({n.right, d + 1});
                     }
                 }
                 scene->statistics.leaves        = leaves;
                 scene->statistics.maximum_depth = depth;
+                interior                        = static_cast<uint32_t>(inner);
             } else {
                 SplitReferences split;
                 if (build && build->split_references) {
@@ -870,6 +858,7 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
                 ref_nodes             = std::move(built.nodes);
                 ref_order             = std::move(built.order);
                 node_count            = built.node_count;
+                interior              = built_interior(node_count);
                 scene->statistics.leaves        = built.leaves;
                 scene->statistics.maximum_depth = built.maximum_depth;
                 scene->build_seconds  = built.seconds;
@@ -889,7 +878,7 @@ std::unique_ptr<Scene> create_scene(const mr_scene_desc& desc, const mr_bvh_desc
         // ---- traversal layout: 4-wide nodes collapsed from the binary tree ----
         uint32_t wide_count = 0;
         if (prims) {
-            WideTree wide = collapse_tree(ref_nodes.ptr, node_count, stream);
+            WideTree wide = collapse_tree(ref_nodes.ptr, interior, stream);
             scene->nodes  = std::move(wide.nodes);
             wide_count    = wide.count;
             scene->tris.allocate(3ull * slots);

@@ -170,7 +170,11 @@ struct WideTree {
     uint32_t             root_count = 0;  // primitives when the root is a leaf (then no nodes)
     float                lo[3] = {}, hi[3] = {};
 };
-WideTree collapse_tree(const mr_bvh_node* nodes, uint32_t node_count, cudaStream_t stream);
+// `interior`: how many interior nodes a walk from the root meets. A subtree that an imported tree enters
+// from several parents counts, and is collapsed, once for each.
+WideTree collapse_tree(const mr_bvh_node* nodes, uint32_t interior, cudaStream_t stream);
+// The same for a tree of `node_count` nodes of the builder's.
+inline uint32_t built_interior(uint32_t node_count) { return node_count / 2; }
 // Sets kTriLeafEnd on the last triangle slot of every leaf of a binary tree.
 void mark_leaf_ends(const mr_bvh_node* nodes, uint32_t node_count, float4* tris, cudaStream_t stream);
 float determinant3(const float* m);

@@ -174,3 +174,25 @@ def test_visit_bound_is_the_same_on_every_route(api, bead_scenes, paths, decoys)
             assert not (out if out.dtype == bool else out["primitive"] != 0xffffffff).any()
         else:
             np.testing.assert_array_equal(out, np.full((paths, 3), 0.5, np.float32))
+
+
+@pytest.mark.parametrize("levels", [1, 2, 3, 8])
+def test_subtrees_of_several_parents(api, levels):
+    """Both children of each of `levels` nodes are the next one, so a walk meets 2^levels - 1 interior
+    nodes of which the import holds `levels`: the wide tree has a node for each time one is met."""
+    triangles = np.array([[(-1, -1, z), (3, -1, z), (-1, 3, z)] for z in (1.0, 2.0)])
+    plain = imported(api, triangles, (0, 1))
+    nodes = [((-1, -1, 1), (3, 3, 2), k + 1, k + 1, 0) for k in range(levels - 1)]
+    nodes += [((-1, -1, 1), (3, 3, 2), levels, levels + 1, 0),
+              ((-1, -1, 1), (3, 3, 1), 0, 0, 1), ((-1, -1, 2), (3, 3, 2), 1, 0, 1)]
+    packed, order = np.array(nodes, NODE), np.arange(2, dtype=np.uint32)
+    desc = _abi.BvhDesc(C.cast(packed.ctypes.data, C.POINTER(_abi.BvhNode)), len(packed),
+                        order.ctypes.data_as(C.POINTER(C.c_uint32)), 2)
+    scene = api.Scene(plain.snapshot, desc)
+    assert scene.statistics()["leaves"] == 2 ** levels
+    rng = np.random.default_rng(2)
+    d = np.column_stack([rng.uniform(-1, 1, (1000, 2)), np.ones(1000)])
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    o = np.zeros_like(d)
+    np.testing.assert_array_equal(scene.intersect(o, d)[0], plain.intersect(o, d)[0])
+    np.testing.assert_array_equal(scene.occluded(o, d)[0], plain.occluded(o, d)[0])

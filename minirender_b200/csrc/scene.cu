@@ -130,10 +130,10 @@ __global__ void collapse_count_kernel(const mr_bvh_node* nodes, const uint32_t* 
     int n    = 2;
     while (n < 4) {
         int   best = -1;
-        float area = -1.0f;
-        for (int i = 0; i < n; ++i) {
+        float area = 0;
+        for (int i = 0; i < n; ++i) {  // an interior child is opened whatever its area (NaN: an infinite box)
             const mr_bvh_node& child = nodes[c[i]];
-            if (child.count == 0 && node_area(child) > area) {
+            if (child.count == 0 && (best < 0 || node_area(child) > area)) {
                 area = node_area(child);
                 best = i;
             }
@@ -374,17 +374,22 @@ WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t interior, cudaStre
         out.hi[a] = root.maximum[a];
     }
     out.root_count = root.count;
-    out.nodes.allocate(std::max<uint32_t>(1, interior) * kWideNode);
-    out.children.allocate(std::max<uint32_t>(1, interior));
+    // Wide nodes at most: one with four children stands for three interior nodes, one with fewer, which
+    // are all leaves, for one or two. Where W have four, they have at most 4 W interior children, so at
+    // most 3 W + 1 have fewer. (Space for `interior` nodes would be half as much again, 192 bytes for
+    // each interior node.)
+    const uint32_t capacity = static_cast<uint32_t>((2ull * interior + 1) / 3);
+    out.nodes.allocate(std::max<uint32_t>(1, capacity) * kWideNode);
+    out.children.allocate(std::max<uint32_t>(1, capacity));
     if (interior == 0) {
         return out;
     }
     DeviceBuffer<uint32_t> roots[2], counts, offsets, scratch;
-    roots[0].allocate(interior);
-    roots[1].allocate(interior);
-    counts.allocate(interior);
-    offsets.allocate(interior);
-    scratch.allocate(scan_scratch_size(interior));
+    roots[0].allocate(capacity);
+    roots[1].allocate(capacity);
+    counts.allocate(capacity);
+    offsets.allocate(capacity);
+    scratch.allocate(scan_scratch_size(capacity));
     MR_CUDA(cudaMemsetAsync(roots[0].ptr, 0, sizeof(uint32_t), stream));  // the root
     // Levels run from counts on the device, a few at a time between the host's looks at them: at
     // most 4^level nodes each, blocks beyond a level's own count leave at once. A wide level holds at
@@ -404,8 +409,8 @@ WideTree collapse_tree(const mr_bvh_node* ref_nodes, uint32_t interior, cudaStre
         collapse_write_kernel<<<(bound + 127) / 128, 128, 0, stream>>>(ref_nodes, out.children.ptr,
                                                                        levels.ptr + level, offsets.ptr,
                                                                        out.nodes.ptr, roots[(level + 1) & 1].ptr);
-        const bool full = bound == interior;
-        bound           = static_cast<uint32_t>(std::min<uint64_t>(4ull * bound, interior));
+        const bool full = bound == capacity;
+        bound           = static_cast<uint32_t>(std::min<uint64_t>(4ull * bound, capacity));
         look            = full ? look - 1 : look;  // the first levels are full ones: no need to look
         if (look == 0 || level + 1 == kMaxLevels) {
             CollapseLevel next{};

@@ -196,3 +196,30 @@ def test_subtrees_of_several_parents(api, levels):
     o = np.zeros_like(d)
     np.testing.assert_array_equal(scene.intersect(o, d)[0], plain.intersect(o, d)[0])
     np.testing.assert_array_equal(scene.occluded(o, d)[0], plain.occluded(o, d)[0])
+
+
+@pytest.mark.parametrize("triangles", [3, 5, 33, 300])
+def test_infinite_flat_boxes(api, triangles):
+    """Interior boxes without bounds in x and y and of no extent in z have no comparable area: the collapse
+    opens them all the same."""
+    rng = np.random.default_rng(triangles)
+    corners = rng.uniform(-1, 1, (triangles, 3, 2))
+    corners = np.concatenate([corners, np.ones((triangles, 3, 1))], 2)
+
+    def halves(begin, end):
+        middle = (begin + end) // 2
+        return begin if end - begin == 1 else (halves(begin, middle), halves(middle, end))
+
+    plain = imported(api, corners, halves(0, triangles))
+    nodes, order, count = plain.export_bvh()
+    packed = np.frombuffer(nodes, NODE)[:count].copy()
+    inner = packed["count"] == 0
+    inner[0] = False  # the scene's bounds
+    packed["minimum"][inner, :2], packed["maximum"][inner, :2] = -np.inf, np.inf
+    desc = _abi.BvhDesc(C.cast(packed.ctypes.data, C.POINTER(_abi.BvhNode)), count,
+                        order.ctypes.data_as(C.POINTER(C.c_uint32)), triangles)
+    scene = api.Scene(plain.snapshot, desc)
+    d = np.column_stack([rng.uniform(-1, 1, (4000, 2)), np.ones(4000)])
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    o = np.zeros_like(d)
+    np.testing.assert_array_equal(scene.intersect(o, d)[0], plain.intersect(o, d)[0])

@@ -445,9 +445,15 @@ void session_run(mr_session* s, const Scene* scene, IntegratorParams params, mr_
             {
                 std::unique_lock<std::mutex> lock(s->control);
                 if (s->pause_requested && !s->cancel_requested) {
-                    s->state = MR_STATE_PAUSED;
-                    s->changed.notify_all();
-                    s->changed.wait(lock, [&] { return !s->pause_requested || s->cancel_requested; });
+                    // Parked. A resume with another pause before this thread has looked leaves the
+                    // state at pausing: it is paused again.
+                    do {
+                        s->state = MR_STATE_PAUSED;
+                        s->changed.notify_all();
+                        s->changed.wait(lock, [&] {
+                            return !s->pause_requested || s->cancel_requested || s->state != MR_STATE_PAUSED;
+                        });
+                    } while (s->pause_requested && !s->cancel_requested);
                     if (!s->cancel_requested) {
                         s->state = MR_STATE_RUNNING;
                     }

@@ -7,7 +7,9 @@
 //   visit   lanes at an interior node test its four children;
 //   leaf    lanes holding a leaf test one of its triangles.
 // Visit or leaf goes to the larger group. A lane postpones the leaf it reaches and keeps descending
-// until it meets a second one, so most lanes can do either.
+// until it meets a second one, so most lanes can do either. (Persistent warps that fetch rays by a vote
+// and a postponed leaf per lane: Aila and Laine, "Understanding the Efficiency of Ray Traversal on
+// GPUs", HPG 2009.)
 //
 // Against one fetch of 32 rays that a warp traces to the end of the slowest, a step runs 18 lanes of
 // 32 where it ran 11 (half of the lane slots had waited for the slowest ray of their fetch, and
@@ -183,7 +185,7 @@ __device__ __forceinline__ void stream_rays(Io& io, uint32_t n, uint32_t* work, 
     int            node = kNoNode, leaf = 0;
     float          tmin = 0;
     NearestHit     hit{0, kNone};
-    StreamRay      ray{};
+    StreamRay      ray;
     uint32_t       next = 0, end = 0;  // the rest of the warp's chunk
     int            refill = kRefill;  // 32 once the queue is empty
     int2           deep[kDeepSize];

@@ -309,8 +309,9 @@ class Server {
     }
 
     // Submits the jobs together: the controller sees all of them when it packs the next wave. One at
-    // a time, it packed a wave of the first few it happened to see, of a depth that needed a graph of
-    // its own (24 preview jobs: 7 ms, or 20 ms when it did).
+    // a time, it packed a wave of the first few it happened to see. 24 preview jobs, median of 300 calls:
+    // 7.5 ms one at a time, 6.9 ms together, both with calls of up to 85 ms among them; a shape's first
+    // call, which makes its graphs, takes 20 ms either way.
     std::vector<uint64_t> submit_all(std::vector<std::unique_ptr<Job>> jobs) {
         std::vector<uint64_t>       ids;
         std::lock_guard<std::mutex> lock(mutex_);

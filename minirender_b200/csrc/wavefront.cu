@@ -1752,7 +1752,6 @@ void render_frame(const Scene& scene, const IntegratorParams& params, const mr_r
     }
 }
 
-// Per-path radiance of an explicit wave (trace_paths / sample_pixels).
 // Loads the kernels of a wave of whole paths from rays: under lazy loading a kernel's first use places
 // its code in device memory.
 void load_path_kernels() {
@@ -1767,6 +1766,7 @@ void load_path_kernels() {
     load(copy_radiance_kernel);
 }
 
+// Per-path radiance of an explicit wave (trace_paths / sample_pixels).
 void copy_path_radiance(Workspace& ws, uint32_t count, float* device_out, cudaStream_t stream) {
     copy_radiance_kernel<<<(count + 255) / 256, 256, 0, stream>>>(ws.state.radiance, count, device_out);
     MR_CUDA(cudaGetLastError());

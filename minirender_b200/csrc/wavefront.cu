@@ -363,6 +363,7 @@ __device__ __forceinline__ void shadow_item(const KernelArgs& a, const DeviceSce
 
 // Queue items of stream_rays: extension rays (SHADOW = false) or shadow segments of a wave's paths.
 template <bool SHADOW, bool MEDIA, bool BATCH> struct QueueIo {
+    static constexpr bool kBatch = BATCH;
     const KernelArgs& a;
     const uint32_t*   queue;
     uint32_t*         bins;
